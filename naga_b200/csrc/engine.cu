@@ -7,6 +7,7 @@
 // init_domain), simulation_observers/density_observer.cuh:62-113 (probes).
 #include "common.cuh"
 #include "scene_dev.hpp"
+#include "scratch.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -109,12 +110,15 @@ struct naga_scene {
     template <class T>
     int alloc(T** p, int64_t count) {
         size_t b = sizeof(T) * (size_t)std::max<int64_t>(count, 1);
-        cudaError_t e = cudaMalloc((void**)p, b);
+        // from the library's pool, ordered on the scene's stream: a scene has
+        // about 30 buffers, and cudaMalloc and cudaFree of them took 9 of the
+        // 24 ms of a 100k-node request (creation, ten steps, release)
+        cudaError_t e = scratch_malloc(p, b, stream);
         if (e != cudaSuccess) {
             *p = nullptr;
             cudaGetLastError();
             return set_error(e == cudaErrorMemoryAllocation ? NAGA_ENOMEM : NAGA_ECUDA,
-                             std::string("naga_scene_create: cudaMalloc: ") + cudaGetErrorString(e));
+                             std::string("naga_scene_create: allocation: ") + cudaGetErrorString(e));
         }
         allocs.push_back((void*)*p);
         bytes += (int64_t)b;
@@ -148,8 +152,7 @@ struct naga_batch {
     int scenes_cap = 0;
     ListCopy* d_copies = nullptr;
     int copies_cap = 0;
-    void* h_stage = nullptr;  // page-locked staging of the scene and copy tables
-    size_t stage_cap = 0;
+    std::vector<char> stage;  // host copy of the scene and copy tables
 
     void free_graph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -159,16 +162,14 @@ struct naga_batch {
     }
     void free_tables() {
         free_graph();
-        if (d_scenes) cudaFree(d_scenes);
-        if (d_items) cudaFree(d_items);
-        if (d_copies) cudaFree(d_copies);
-        if (h_stage) cudaFreeHost(h_stage);
+        if (d_scenes) cudaFreeAsync(d_scenes, stream);
+        if (d_items) cudaFreeAsync(d_items, stream);
+        if (d_copies) cudaFreeAsync(d_copies, stream);
         d_scenes = nullptr;
         d_items = nullptr;
         d_copies = nullptr;
-        h_stage = nullptr;
         d_all = d_all_mt = d_fluid = d_edge = d_pml = nullptr;
-        items_cap = stage_cap = 0;
+        items_cap = 0;
         scenes_cap = copies_cap = 0;
     }
 };
@@ -296,11 +297,11 @@ int rpim_tables(naga_scene* s, const float* pts, const float* qry_host, int64_t 
     float* dq = nullptr;
     double* dqd = nullptr;
     double* dw = nullptr;
-    NAGA_CUDA_TRY(cudaMallocAsync(&didx, sizeof(uint32_t) * nq * kk, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&dd2, sizeof(float) * nq * kk, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&dq, sizeof(float) * nq * D, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&dqd, sizeof(double) * nq * D, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&dw, sizeof(double) * nq * kk, st));
+    NAGA_CUDA_TRY(scratch_malloc(&didx, sizeof(uint32_t) * nq * kk, st));
+    NAGA_CUDA_TRY(scratch_malloc(&dd2, sizeof(float) * nq * kk, st));
+    NAGA_CUDA_TRY(scratch_malloc(&dq, sizeof(float) * nq * D, st));
+    NAGA_CUDA_TRY(scratch_malloc(&dqd, sizeof(double) * nq * D, st));
+    NAGA_CUDA_TRY(scratch_malloc(&dw, sizeof(double) * nq * kk, st));
     std::vector<double> qd(nq * D);
     for (int64_t t = 0; t < nq * D; ++t) qd[t] = qry_host[t];
     NAGA_CUDA_TRY(cudaMemcpyAsync(dq, qry_host, sizeof(float) * nq * D, cudaMemcpyHostToDevice, st));
@@ -521,8 +522,8 @@ int scene_setup(naga_scene* s) {
         const int nf = (int)s->items_fluid.size();
         WorkItem* ditems = nullptr;
         uint8_t* dflag = nullptr;
-        NAGA_CUDA_TRY(cudaMallocAsync(&ditems, sizeof(WorkItem) * nf, st));
-        NAGA_CUDA_TRY(cudaMallocAsync(&dflag, nf, st));
+        NAGA_CUDA_TRY(scratch_malloc(&ditems, sizeof(WorkItem) * nf, st));
+        NAGA_CUDA_TRY(scratch_malloc(&dflag, nf, st));
         std::vector<uint8_t> flag(nf, 0);
         cudaError_t e = cudaMemcpyAsync(ditems, s->items_fluid.data(), sizeof(WorkItem) * nf, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) {
@@ -543,8 +544,8 @@ int scene_setup(naga_scene* s) {
             WorkItem* dpi = nullptr;
             uint32_t* dk = nullptr;
             std::vector<uint32_t> km(np, 0);
-            e = cudaMallocAsync(&dpi, sizeof(WorkItem) * np, st);
-            if (e == cudaSuccess) e = cudaMallocAsync(&dk, sizeof(uint32_t) * np, st);
+            e = scratch_malloc(&dpi, sizeof(WorkItem) * np, st);
+            if (e == cudaSuccess) e = scratch_malloc(&dk, sizeof(uint32_t) * np, st);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(dpi, s->items_pml.data(), sizeof(WorkItem) * np, cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess) {
@@ -604,15 +605,17 @@ int batch_rebuild(naga_batch* b) {
     for (int l = 0; l < 5; ++l) base[l + 1] = base[l] + n[l];
     for (int l = 0; l < 5; ++l)
         if (n[l] > 0x7fffffff) return set_error(NAGA_EINVAL, "batch: more than 2^31 - 1 work items in one list");
-    // grow the device tables (cudaFree waits for the device, so only here)
+    // grow the device tables (on the batch's stream, like everything that
+    // reads them)
     auto grow = [&](auto** p, auto& cap, int64_t need) -> int {
         if (need <= (int64_t)cap && *p) return NAGA_OK;
-        if (*p) cudaFree(*p);
+        if (*p) cudaFreeAsync(*p, b->stream);
         *p = nullptr;
         const int64_t c = std::max<int64_t>(need + need / 4, 16);
         using T = typename std::remove_pointer<typename std::remove_reference<decltype(*p)>::type>::type;
-        cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (size_t)c);
+        cudaError_t e = scratch_malloc(p, sizeof(T) * (size_t)c, b->stream);
         if (e != cudaSuccess) {
+            *p = nullptr;
             cudaGetLastError();
             cap = 0;
             return set_error(e == cudaErrorMemoryAllocation ? NAGA_ENOMEM : NAGA_ECUDA,
@@ -638,14 +641,8 @@ int batch_rebuild(naga_batch* b) {
     if ((rc = grow(&b->d_scenes, b->scenes_cap, std::max(ns, 1)))) return rc;
     if ((rc = grow(&b->d_copies, b->copies_cap, std::max<int64_t>((int64_t)copies.size(), 1)))) return rc;
     const size_t sb = sizeof(SceneDev) * ns, cb = sizeof(ListCopy) * copies.size();
-    if (sb + cb > b->stage_cap) {
-        if (b->h_stage) cudaFreeHost(b->h_stage);
-        b->h_stage = nullptr;
-        b->stage_cap = 0;
-        NAGA_CUDA_TRY(cudaMallocHost(&b->h_stage, (sb + cb) * 5 / 4 + 256));
-        b->stage_cap = (sb + cb) * 5 / 4 + 256;
-    }
-    char* stage = (char*)b->h_stage;
+    if (sb + cb > b->stage.size()) b->stage.resize(sb + cb);
+    char* stage = b->stage.data();
     for (int t = 0; t < ns; ++t) std::memcpy(stage + sizeof(SceneDev) * t, &b->members[t]->dev, sizeof(SceneDev));
     if (cb) std::memcpy(stage + sb, copies.data(), cb);
     if (sb) NAGA_CUDA_TRY(cudaMemcpyAsync(b->d_scenes, stage, sb, cudaMemcpyHostToDevice, b->stream));
@@ -810,7 +807,7 @@ extern "C" int naga_scene_destroy(naga_scene* s) {
     if (s->owner) naga_batch_remove(s->owner, s);
     if (s->solo) naga_batch_destroy(s->solo);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (void* p : s->allocs) cudaFree(p);
+    for (void* p : s->allocs) cudaFreeAsync(p, s->stream);
     if (s->src_slot) cudaFree(s->src_slot);
     if (s->src_vals) cudaFree(s->src_vals);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -886,7 +883,7 @@ void release(naga_scene* s, void* p) {
     auto it = std::find(s->allocs.begin(), s->allocs.end(), p);
     if (it == s->allocs.end()) return;
     s->allocs.erase(it);
-    cudaFree(p);
+    cudaFreeAsync(p, s->stream);
 }
 }  // namespace
 
@@ -906,6 +903,9 @@ extern "C" int naga_scene_add_probe(naga_scene* s, const float* xyz, int* index)
     float* ring = nullptr;
     const int64_t cap = s->dev.probe_cap;
     if (!rc) rc = s->alloc(&ring, cap * np);
+    // the allocations are ordered on the scene's own stream
+    if (!rc && cudaStreamSynchronize(s->stream) != cudaSuccess)
+        rc = set_error(NAGA_ECUDA, "naga_scene_add_probe: allocation");
     if (rc) {
         s->probe_xyz.resize((size_t)np_old * D);
         release(s, pidx);

@@ -19,11 +19,11 @@
 // that does not already touch the edge of the grid.
 #include "common.cuh"
 #include "scene_dev.hpp"
+#include "scratch.hpp"
 
 #include <cstring>
 
 #include <cub/device/device_scan.cuh>
-#include <cuda.h>
 
 #include <cmath>
 #include <mutex>
@@ -330,10 +330,10 @@ int knn_run(const float* src, const int64_t* h_src_off, int nclouds, const float
         fail(e, what);         \
         goto done;             \
     }
-    KTRY(cudaMallocAsync(&d_off, sizeof(int64_t) * (nclouds + 1), st), "alloc");
+    KTRY(scratch_malloc(&d_off, sizeof(int64_t) * (nclouds + 1), st), "alloc");
     KTRY(cudaMemcpyAsync(d_off, h_src_off, sizeof(int64_t) * (nclouds + 1), cudaMemcpyHostToDevice, st), "copy");
     if (h_q_off) {
-        KTRY(cudaMallocAsync(&d_qoff, sizeof(int64_t) * (nclouds + 1), st), "alloc");
+        KTRY(scratch_malloc(&d_qoff, sizeof(int64_t) * (nclouds + 1), st), "alloc");
         KTRY(cudaMemcpyAsync(d_qoff, h_q_off, sizeof(int64_t) * (nclouds + 1), cudaMemcpyHostToDevice, st), "copy");
     }
     for (int c = 0; c < nclouds; ++c)
@@ -341,7 +341,7 @@ int knn_run(const float* src, const int64_t* h_src_off, int nclouds, const float
             hb[c * 6 + d] = 0x7fffffff;
             hb[c * 6 + 3 + d] = (int)0x80000000;
         }
-    KTRY(cudaMallocAsync(&d_bbox, sizeof(int) * 6 * nclouds, st), "alloc");
+    KTRY(scratch_malloc(&d_bbox, sizeof(int) * 6 * nclouds, st), "alloc");
     KTRY(cudaMemcpyAsync(d_bbox, hb.data(), sizeof(int) * 6 * nclouds, cudaMemcpyHostToDevice, st), "copy");
     if (total > 0) {
         int blocks = (int)std::min<int64_t>((total + 255) / 256, 4 * 148 * 8);
@@ -381,21 +381,21 @@ int knn_run(const float* src, const int64_t* h_src_off, int nclouds, const float
         g.n = n;
         ncell += cells;
     }
-    KTRY(cudaMallocAsync(&d_grids, sizeof(CloudGrid) * nclouds, st), "alloc");
+    KTRY(scratch_malloc(&d_grids, sizeof(CloudGrid) * nclouds, st), "alloc");
     KTRY(cudaMemcpyAsync(d_grids, grids.data(), sizeof(CloudGrid) * nclouds, cudaMemcpyHostToDevice, st), "copy");
-    KTRY(cudaMallocAsync(&d_counts, sizeof(unsigned) * (ncell + 1), st), "alloc");
-    KTRY(cudaMallocAsync(&d_start, sizeof(unsigned) * (ncell + 1), st), "alloc");
-    KTRY(cudaMallocAsync(&d_fill, sizeof(unsigned) * (ncell + 1), st), "alloc");
+    KTRY(scratch_malloc(&d_counts, sizeof(unsigned) * (ncell + 1), st), "alloc");
+    KTRY(scratch_malloc(&d_start, sizeof(unsigned) * (ncell + 1), st), "alloc");
+    KTRY(scratch_malloc(&d_fill, sizeof(unsigned) * (ncell + 1), st), "alloc");
     KTRY(cudaMemsetAsync(d_counts, 0, sizeof(unsigned) * (ncell + 1), st), "memset");
     KTRY(cudaMemsetAsync(d_fill, 0, sizeof(unsigned) * (ncell + 1), st), "memset");
-    KTRY(cudaMallocAsync(&d_sorted, sizeof(float4) * std::max<int64_t>(total, 1), st), "alloc");
+    KTRY(scratch_malloc(&d_sorted, sizeof(float4) * std::max<int64_t>(total, 1), st), "alloc");
     if (total > 0) {
         int blocks = (int)std::min<int64_t>((total + 255) / 256, 4 * 148 * 8);
         count_kernel<D><<<blocks, 256, 0, st>>>(src, d_off, nclouds, total, d_grids, d_counts);
         KTRY(cudaGetLastError(), "count kernel");
     }
     KTRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_counts, d_start, ncell + 1, st), "scan size");
-    KTRY(cudaMallocAsync(&d_tmp, tmp_bytes, st), "alloc");
+    KTRY(scratch_malloc(&d_tmp, tmp_bytes, st), "alloc");
     KTRY(cub::DeviceScan::ExclusiveSum(d_tmp, tmp_bytes, d_counts, d_start, ncell + 1, st), "scan");
     if (total > 0) {
         int blocks = (int)std::min<int64_t>((total + 255) / 256, 4 * 148 * 8);
@@ -467,29 +467,6 @@ struct NoAllocScratch {
 };
 
 static __device__ __align__(256) unsigned char g_knn_scratch[sizeof(NoAllocScratch)];
-
-// Unique id of the calling thread's current context (cuCtxGetId through the
-// runtime's driver entry points, so the library needs no libcuda link);
-// false when it cannot be had (no current context, an older driver).
-bool current_context_id(unsigned long long* id) {
-    using GetCurrent = CUresult (*)(CUcontext*);
-    using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", (void**)&get_current, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            get_current = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", (void**)&get_id, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            get_id = nullptr;
-    });
-    CUcontext ctx = nullptr;
-    if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx) return false;
-    return get_id(ctx, id) == CUDA_SUCCESS;
-}
 
 // device address of g_knn_scratch in the current context: looked up once
 // per device and context, and again when the device's context changed (a

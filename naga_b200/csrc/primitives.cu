@@ -11,6 +11,7 @@
 // serve callers of the primitives (the C++ facade's classes of the same
 // names).
 #include "common.cuh"
+#include "scratch.hpp"
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -222,7 +223,7 @@ extern "C" int naga_segmentation_shape(const float* pts, int64_t n, int dim, int
         hb[d] = 0x7fffffff;
         hb[3 + d] = (int)0x80000000;
     }
-    NAGA_CUDA_TRY(cudaMallocAsync(&d_b, sizeof hb, st));
+    NAGA_CUDA_TRY(scratch_malloc(&d_b, sizeof hb, st));
     NAGA_CUDA_TRY(cudaMemcpyAsync(d_b, hb, sizeof hb, cudaMemcpyHostToDevice, st));
     const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 8);
     if (dim == 2)
@@ -272,9 +273,9 @@ extern "C" int naga_segmentation_build(const float* pts, int64_t n, int dim, con
     size_t tmp_scan = 0, tmp_sort = 0;
     int bits = 1;
     while (bits < 32 && (((int64_t)1 << bits) < cells)) ++bits;
-    NAGA_CUDA_TRY(cudaMallocAsync(&cell, sizeof(uint32_t) * n, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&cell_sorted, sizeof(uint32_t) * n, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&iota, sizeof(uint32_t) * n, st));
+    NAGA_CUDA_TRY(scratch_malloc(&cell, sizeof(uint32_t) * n, st));
+    NAGA_CUDA_TRY(scratch_malloc(&cell_sorted, sizeof(uint32_t) * n, st));
+    NAGA_CUDA_TRY(scratch_malloc(&iota, sizeof(uint32_t) * n, st));
     NAGA_CUDA_TRY(cudaMemsetAsync(sizes, 0, sizeof(uint32_t) * cells, st));
     const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 8);
     if (dim == 2)
@@ -290,7 +291,7 @@ extern "C" int naga_segmentation_build(const float* pts, int64_t n, int dim, con
     NAGA_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_scan, sizes, offsets, cells, st));
     NAGA_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_sort, cell, cell_sorted, iota, indices, n, 0, bits,
                                                   st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&tmp, std::max(tmp_scan, tmp_sort), st));
+    NAGA_CUDA_TRY(scratch_malloc(&tmp, std::max(tmp_scan, tmp_sort), st));
     NAGA_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_scan, sizes, offsets, cells, st));
     NAGA_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_sort, cell, cell_sorted, iota, indices, n, 0, bits, st));
     NAGA_CUDA_TRY(cudaFreeAsync(tmp, st));
@@ -311,8 +312,8 @@ extern "C" int naga_rbf_weights_f32(const float* src, int64_t n, int dim, const 
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t nq = ngroups * group;
     double *q64 = nullptr, *w64 = nullptr;
-    NAGA_CUDA_TRY(cudaMallocAsync(&q64, sizeof(double) * nq * dim, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&w64, sizeof(double) * nq * k, st));
+    NAGA_CUDA_TRY(scratch_malloc(&q64, sizeof(double) * nq * dim, st));
+    NAGA_CUDA_TRY(scratch_malloc(&w64, sizeof(double) * nq * k, st));
     const int b1 = (int)std::min<int64_t>((nq * dim + 255) / 256, (int64_t)sm_count() * 8);
     widen_kernel<<<b1, 256, 0, st>>>(qry, q64, nq * dim);
     NAGA_CUDA_TRY(cudaGetLastError());

@@ -16,6 +16,7 @@
 // system.
 #include "warp_lu.cuh"
 #include "scene_dev.hpp"
+#include "scratch.hpp"
 
 #include <algorithm>
 #include <mutex>
@@ -801,7 +802,7 @@ int rbf_weights_device(const float* src, int64_t nsrc, int dim, const uint32_t* 
     const int wpb = warps_per_block_for(per_warp);
     if (wpb < 1) return set_error(NAGA_EINVAL, "naga_rbf_weights: system too large");
     int* d_status = nullptr;
-    NAGA_CUDA_TRY(cudaMallocAsync(&d_status, 2 * sizeof(int), st));
+    NAGA_CUDA_TRY(scratch_malloc(&d_status, 2 * sizeof(int), st));
     NAGA_CUDA_TRY(cudaMemsetAsync(d_status, 0, 2 * sizeof(int), st));
     const int blocks = (int)std::min<int64_t>((ngroups + wpb - 1) / wpb, (int64_t)sm_count() * 32);
     const size_t smem = per_warp * wpb;
@@ -856,15 +857,15 @@ int divergence_build_device(const float* pts, int64_t n, int dim, int k, int sha
     int* d_status = nullptr;
     const int64_t batch = 16384;
     const int64_t nb = (n + batch - 1) / batch;
-    NAGA_CUDA_TRY(cudaMallocAsync(&d2, sizeof(float) * n * k, st));
+    NAGA_CUDA_TRY(scratch_malloc(&d2, sizeof(float) * n * k, st));
     int rc = knn_device(pts, n, pts, n, dim, k, idx, d2, st);
     if (rc) {
         cudaFreeAsync(d2, st);
         return rc;
     }
-    NAGA_CUDA_TRY(cudaMallocAsync(&nn, sizeof(double) * n, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&sp, sizeof(double) * nb, st));
-    NAGA_CUDA_TRY(cudaMallocAsync(&d_status, 2 * sizeof(int), st));
+    NAGA_CUDA_TRY(scratch_malloc(&nn, sizeof(double) * n, st));
+    NAGA_CUDA_TRY(scratch_malloc(&sp, sizeof(double) * nb, st));
+    NAGA_CUDA_TRY(scratch_malloc(&d_status, 2 * sizeof(int), st));
     NAGA_CUDA_TRY(cudaMemsetAsync(d_status, 0, 2 * sizeof(int), st));
     {
         const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 8);
