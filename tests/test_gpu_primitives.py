@@ -41,6 +41,49 @@ def test_knn_bit_exact(naga, oracle, dim, k):
     assert np.array_equal(_np(d2), od)
 
 
+def _awkward_cloud(kind, dim, rng):
+    """Clouds whose density misleads the search's first radius, or that it
+    leaves to the shell walk."""
+    u = lambda n: rng.random((n, dim))  # noqa: E731
+    if kind == "clusters":  # most points in a few tight clumps of a wide box
+        return np.concatenate([u(200), *(u(1) + 1e-3 * rng.standard_normal((700, dim)) for _ in range(4))])
+    if kind == "sheet":  # one axis without extent
+        p = u(3000)
+        p[:, -1] = 0.25
+        return p
+    if kind == "line":
+        p = np.full((2000, dim), 0.5)
+        p[:, 0] = rng.random(2000)
+        return p
+    if kind == "stacks":  # 150 copies of each of 20 points: more ties than the collected keys
+        return np.repeat(u(20), 150, 0)
+    if kind == "lattice":  # exact distance ties at every radius
+        m = 14 if dim == 3 else 50
+        return np.stack(np.meshgrid(*[np.arange(m)] * dim, indexing="ij"), -1).reshape(-1, dim) / 16.0
+    if kind == "far":  # large coordinates, coarse FP32 spacing
+        return 1e5 + u(3000)
+    return u(70)  # "few": barely more points than the largest k
+
+
+@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "lattice", "far", "few"])
+@pytest.mark.parametrize("dim,k", [(2, 16), (3, 32), (3, 33), (2, 64)])
+def test_knn_awkward_clouds(naga, oracle, kind, dim, k):
+    """Self and free queries (inside, beside and far outside the cloud)
+    against the oracle, bit for bit: the radius search, its rescaling, and
+    the shell walk behind it."""
+    rng = np.random.default_rng(77)
+    pts = _awkward_cloud(kind, dim, rng).astype(np.float32)
+    span = pts.max(0) - pts.min(0)
+    box = pts.min(0) + span * (rng.random((200, dim)) * 3 - 1)
+    qry = np.concatenate([box, pts[:50], pts.min(0) - 40 * span.max() * rng.random((5, dim))]).astype(np.float32)
+    src = _t(pts)
+    for q, t in ((pts, src), (qry, _t(qry))):
+        idx, d2 = naga.knn(src, t, k)
+        oi, od = oracle.knn(pts, q, k, grid=False)
+        assert np.array_equal(_np(idx).view(np.uint32), oi)
+        assert np.array_equal(_np(d2), od)
+
+
 def test_knn_golden_validation_grid(naga, golden_dir):
     g = json.load(open(os.path.join(golden_dir, "knn_validation_3d.json")))
     n1, h, k = g["grid_size"], np.float32(g["spacing"]), g["k"]
