@@ -128,18 +128,6 @@ __device__ __forceinline__ float cs_f() { return 0.57735026918962576450914878050
 
 // full row (QP floats) of node i, slot order
 template <class L>
-__device__ __forceinline__ void load_row(const float* base, int64_t i, float* v) {
-    const float4* p = reinterpret_cast<const float4*>(base + i * L::QP);
-#pragma unroll
-    for (int c = 0; c < L::QP / 4; ++c) {
-        float4 t = p[c];
-        v[4 * c + 0] = t.x;
-        v[4 * c + 1] = t.y;
-        v[4 * c + 2] = t.z;
-        v[4 * c + 3] = t.w;
-    }
-}
-template <class L>
 __device__ __forceinline__ void store_row(float* base, int64_t i, const float* v) {
     float4* p = reinterpret_cast<float4*>(base + i * L::QP);
 #pragma unroll
@@ -250,217 +238,152 @@ __device__ __forceinline__ void macros(const float* g, float& drho, float* u) {
     for (int d = 0; d < L::D; ++d) u[d] = m[d] * rrho;
 }
 
-// centred equilibrium feq - w of detail/equilibrium_distribution.cuh:41-64:
-// w rho (1 + u.c / cs^2 + (u.c)^2 / (2 cs^4) - u.u) - w
+// centred equilibrium feq - w of detail/equilibrium_distribution.cuh:41-64,
+// w rho (1 + u.c / cs^2 + (u.c)^2 / (2 cs^4) - u.u) - w, of population a and
+// of its opposite (of the rest population: it alone): the terms even and odd
+// in the direction, shared by the two. 1 / cs^2 and 1 / (2 cs^4) are
+// compile-time constants.
 template <class L>
-__device__ __forceinline__ float feq_c(int a, float drho, const float* u) {
+__device__ __forceinline__ void feq_pair(int a, float drho, const float* u, float uu, float* f) {
     using T = Lat<L>;
-    const float cs = cs_f();
-    const float cs2 = cs * cs, cs4 = cs2 * cs2;
-    float uu = u[0] * u[0] + u[1] * u[1];
-    float uc = (float)T::cx(a) * u[0] + (float)T::cy(a) * u[1];
-    if (L::D == 3) {
-        uu += u[2] * u[2];
-        uc += (float)T::cz(a) * u[2];
-    }
-    const float w = T::w(a);
-    // 1 / cs^2 and 1 / (2 cs^4) are compile-time constants: multiplications
-    // instead of 2 x 27 IEEE divisions per feq evaluation (rounding differs
-    // from dividing by at most an ulp of each term)
     constexpr float r_cs2 = (float)(1.0 / ((double)0.57735026918962576451f * 0.57735026918962576451f));
     constexpr float r_2cs4 = 0.5f * r_cs2 * r_cs2;
-    (void)cs4;
-    return w * drho + w * (1.f + drho) * (uc * r_cs2 + (uc * uc) * r_2cs4 - uu);
+    f[0] = f[1] = 0.f;
+    if (a < 0) return;  // two pads
+    float uc = (float)T::cx(a) * u[0] + (float)T::cy(a) * u[1];
+    if (L::D == 3) uc += (float)T::cz(a) * u[2];
+    const float w = T::w(a), wr = w * (1.f + drho);
+    const float even = fmaf(wr, fmaf(uc * uc, r_2cs4, -uu), w * drho), odd = wr * (uc * r_cs2);
+    f[0] = even + odd;
+    f[1] = even - odd;
 }
 
 // ------------------------------------------------------------- collision
 // D3Q27 central-moment collision (detail/d3q27_lattice.cuh:125-378) on
-// centred populations. Central moments K_mnp of f = w + g split into the
-// weight part, a product of 1-D moments M_0 = 1, M_1 = -u, M_2 = 1/3 + u^2
-// (the D3Q27 weights factorise per axis), and the g part. Every moment is
-// carried as K = C + s, with C its value at u = 0 (non-zero only for the
-// even moments) and s small; terms of the k formulas without a velocity
-// factor use s (and rho - 1), where the reference's C contributions cancel
-// exactly, all other terms use K.
-__device__ __forceinline__ void mom1(int m, float u, float& a, float& x) {
-    a = (m == 0) ? 1.f : (m == 1 ? 0.f : 1.f * (1.f / 3.f));
-    x = (m == 0) ? 0.f : (m == 1 ? -u : u * u);
-}
-
-__device__ void collide_d3q27(const float* g, float drho, const float* u, const SceneDev& S, float* delta) {
+// centred populations. Each of the reference's k formulas is the projection of
+// f - f^ on one column of the collision matrix (the orthogonal moment basis,
+// its squared length the formula's divisor), relaxed at the moment's rate,
+// where f^ is the equilibrium whose central moments factorise per axis (1, 0,
+// 1/3): the u-dependent terms of the formulas are the central moments written
+// out in raw ones. So the collision runs on raw moments: three 1-D transforms
+// (sums and differences of three values) to the moments of g, minus those of
+// f^ - w, the basis combinations, and three 1-D evaluations back. Mass and
+// momentum of f - f^ are zero and left out.
+// The moments of f^ - w are (1 + drho) M M M - W W W with M = (1, u, 1/3 + u^2)
+// and W = (1, 0, 1/3): the O(1) parts cancel term by term (M = W + x, x small),
+// so only the small remainders enter the FP32 arithmetic. About 500 operations
+// a node instead of about 2000.
+__device__ __forceinline__ void collide_d3q27(const float* g, float drho, const float* u, const SceneDev& S,
+                                              float* delta) {
     using T = Lat<D3Q27>;
-    // central moments of g by successive 1-D transforms along x, y, z
-    float Tx[3][3][3];  // [m][cy+1][cz+1]
+    float h[3][3][3];
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
+    for (int a = 0; a < 27; ++a) h[T::cx(a) + 1][T::cy(a) + 1][T::cz(a) + 1] = g[a];
+    // values at -1, 0, 1 -> moments 0, 1, 2, along x, y, z
+    auto moments = [](float& m, float& z, float& p) {
+        const float s = p + m, d = p - m;
+        m = z + s;
+        z = d;
+        p = s;
+    };
+    // coefficients of 1, c, c^2 -> values at -1, 0, 1
+    auto values = [](float& c0, float& c1, float& c2) {
+        const float e = c0 + c2, o = c1, z = c0;
+        c0 = e - o;
+        c1 = z;
+        c2 = e + o;
+    };
 #pragma unroll
-        for (int y = 0; y < 3; ++y)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int z = 0; z < 3; ++z) Tx[m][y][z] = 0.f;
+        for (int j = 0; j < 3; ++j) moments(h[0][i][j], h[1][i][j], h[2][i][j]);
 #pragma unroll
-    for (int a = 0; a < 27; ++a) {
-        const float ax = (float)T::cx(a) - u[0];
-        const int y = T::cy(a) + 1, z = T::cz(a) + 1;
-        Tx[0][y][z] += g[a];
-        Tx[1][y][z] += g[a] * ax;
-        Tx[2][y][z] += g[a] * (ax * ax);
-    }
-    float U[3][3][3];  // [m][n][cz+1]
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
+        for (int j = 0; j < 3; ++j) moments(h[i][0][j], h[i][1][j], h[i][2][j]);
 #pragma unroll
-        for (int z = 0; z < 3; ++z) {
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int y = 0; y < 3; ++y) {
-                const float ay = (float)(y - 1) - u[1];
-                const float t = Tx[m][y][z];
-                s0 += t;
-                s1 += t * ay;
-                s2 += t * (ay * ay);
-            }
-            U[m][0][z] = s0;
-            U[m][1][z] = s1;
-            U[m][2][z] = s2;
-        }
-    float Kg[3][3][3];
+        for (int j = 0; j < 3; ++j) moments(h[i][j][0], h[i][j][1], h[i][j][2]);
+    // minus the moments of f^ - w
+    const float W[3] = {1.f, 0.f, 1.f / 3.f};
+    const float X[3][3] = {{0.f, u[0], u[0] * u[0]}, {0.f, u[1], u[1] * u[1]}, {0.f, u[2], u[2] * u[2]}};
 #pragma unroll
     for (int m = 0; m < 3; ++m)
 #pragma unroll
         for (int n = 0; n < 3; ++n) {
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-#pragma unroll
-            for (int z = 0; z < 3; ++z) {
-                const float az = (float)(z - 1) - u[2];
-                const float t = U[m][n][z];
-                s0 += t;
-                s1 += t * az;
-                s2 += t * (az * az);
-            }
-            Kg[m][n][0] = s0;
-            Kg[m][n][1] = s1;
-            Kg[m][n][2] = s2;
-        }
-    // small parts s_mnp = (Kw(u) - C) + Kg and full values K = C + s
-    float sK[3][3][3], K[3][3][3];
-#pragma unroll
-    for (int m = 0; m < 3; ++m)
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
+            // the x, y factors: WW their rest value, XX the small rest
+            const float WW = W[m] * W[n], XX = X[0][m] * (W[n] + X[1][n]) + W[m] * X[1][n];
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
-                float a0, x0, a1, x1, a2, x2;
-                mom1(m, u[0], a0, x0);
-                mom1(n, u[1], a1, x1);
-                mom1(p, u[2], a2, x2);
-                const float e = x0 * ((a1 + x1) * (a2 + x2)) + a0 * (x1 * (a2 + x2) + a1 * x2);
-                sK[m][n][p] = e + Kg[m][n][p];
-                K[m][n][p] = a0 * a1 * a2 + sK[m][n][p];
+                if (m + n + p < 2) continue;
+                const float M = W[p] + X[2][p];
+                const float x = XX * M + WW * X[2][p];
+                h[m][n][p] -= fmaf(drho, fmaf(WW, W[p], x), x);
             }
-    const float rho = 1.f + drho;
-    const float v0 = u[0], v1 = u[1], v2 = u[2];
-    const float v0sq = v0 * v0, v1sq = v1 * v1, v2sq = v2 * v2;
-    // odd moments (C = 0): one value
-    const float Kxy = K[1][1][0], Kxz = K[1][0][1], Kyz = K[0][1][1];
-    const float Kxxy = K[2][1][0], Kxxz = K[2][0][1], Kxyy = K[1][2][0];
-    const float Kyyz = K[0][2][1], Kxzz = K[1][0][2], Kyzz = K[0][1][2];
-    const float Kxyz = K[1][1][1], Kxyzz = K[1][1][2], Kxxyz = K[2][1][1], Kxyyz = K[1][2][1];
-    const float Kxxyzz = K[2][1][2], Kxyyzz = K[1][2][2], Kxxyyz = K[2][2][1];
-    // even moments: full (u terms) and small (constant terms)
-    const float Kxx = K[2][0][0], Kyy = K[0][2][0], Kzz = K[0][0][2];
-    const float Kxxyy = K[2][2][0], Kxxzz = K[2][0][2], Kyyzz = K[0][2][2], Kxxyyzz = K[2][2][2];
-    const float sxx = sK[2][0][0], syy = sK[0][2][0], szz = sK[0][0][2];
-    const float sxxyy = sK[2][2][0], sxxzz = sK[2][0][2], syyzz = sK[0][2][2], sxxyyzz = sK[2][2][2];
-    (void)Kxxyyzz;
-
-    float k[27];
-    k[0] = k[1] = k[2] = k[3] = 0.f;
-    float om = S.om_ab;
-    k[4] = om * (-Kxy * (1.f / 12.f));
-    k[5] = om * (-Kxz * (1.f / 12.f));
-    k[6] = om * (-Kyz * (1.f / 12.f));
-    k[7] = om * (-(sxx - syy) * (1.f / 12.f));
-    k[8] = om * (-(sxx + syy - 2.f * szz) * (1.f / 36.f));
-    k[9] = om * (-(sxx + syy + szz - drho) * (1.f / 18.f));
-    om = S.om_fix[0];
-    k[10] = om * (-(6.f * Kxy * v1 + 3.f * Kxyy + 6.f * Kxz * v2 + 3.f * Kxzz + 3.f * Kyy * v0 + 3.f * Kzz * v0 -
-                    2.f * rho * v0) * (1.f / 72.f));
-    k[11] = om * (-(3.f * Kxx * v1 + 3.f * Kxxy + 6.f * Kxy * v0 + 6.f * Kyz * v2 + 3.f * Kyzz + 3.f * Kzz * v1 -
-                    2.f * rho * v1) * (1.f / 72.f));
-    k[12] = om * (-(3.f * Kxx * v2 + 3.f * Kxxz + 6.f * Kxz * v0 + 3.f * Kyy * v2 + 3.f * Kyyz + 6.f * Kyz * v1 -
-                    2.f * rho * v2) * (1.f / 72.f));
-    om = S.om_fix[1];
-    k[13] = om * (-(2.f * Kxy * v1 + Kxyy - 2.f * Kxz * v2 - Kxzz + Kyy * v0 - Kzz * v0) / 8.f);
-    k[14] = om * (-(Kxx * v1 + Kxxy + 2.f * Kxy * v0 - 2.f * Kyz * v2 - Kyzz - Kzz * v1) / 8.f);
-    k[15] = om * (-(Kxx * v2 + Kxxz + 2.f * Kxz * v0 - Kyy * v2 - Kyyz - 2.f * Kyz * v1) / 8.f);
-    om = S.om_fix[2];
-    k[16] = om * (-(Kxy * v2 + Kxyz + Kxz * v1 + Kyz * v0) / 8.f);
-    om = S.om_fix[3];
-    k[17] = om * (-(3.f * Kxx * v1sq + 3.f * Kxx * v2sq - 4.f * sxx + 6.f * Kxxy * v1 + 3.f * sxxyy +
-                    6.f * Kxxz * v2 + 3.f * sxxzz + 12.f * Kxy * v0 * v1 + 6.f * Kxyy * v0 +
-                    12.f * Kxz * v0 * v2 + 6.f * Kxzz * v0 + 3.f * Kyy * v0sq + 3.f * Kyy * v2sq - 4.f * syy +
-                    6.f * Kyyz * v2 + 3.f * syyzz + 12.f * Kyz * v1 * v2 + 6.f * Kyzz * v1 + 3.f * Kzz * v0sq +
-                    3.f * Kzz * v1sq - 4.f * szz - 2.f * rho * v0sq - 2.f * rho * v1sq - 2.f * rho * v2sq +
-                    3.f * drho) * (1.f / 36.f));
-    om = S.om_fix[4];
-    k[18] = om * (-(3.f * Kxx * v1sq + 3.f * Kxx * v2sq - 4.f * sxx + 6.f * Kxxy * v1 + 3.f * sxxyy +
-                    6.f * Kxxz * v2 + 3.f * sxxzz + 12.f * Kxy * v0 * v1 + 6.f * Kxyy * v0 +
-                    12.f * Kxz * v0 * v2 + 6.f * Kxzz * v0 + 3.f * Kyy * v0sq - 6.f * Kyy * v2sq + 2.f * syy -
-                    12.f * Kyyz * v2 - 6.f * syyzz - 24.f * Kyz * v1 * v2 - 12.f * Kyzz * v1 + 3.f * Kzz * v0sq -
-                    6.f * Kzz * v1sq + 2.f * szz - 2.f * rho * v0sq + rho * v1sq + rho * v2sq) * (1.f / 72.f));
-    k[19] = om * (-(3.f * Kxx * v1sq - 3.f * Kxx * v2sq + 6.f * Kxxy * v1 + 3.f * sxxyy - 6.f * Kxxz * v2 -
-                    3.f * sxxzz + 12.f * Kxy * v0 * v1 + 6.f * Kxyy * v0 - 12.f * Kxz * v0 * v2 -
-                    6.f * Kxzz * v0 + 3.f * Kyy * v0sq - 2.f * syy - 3.f * Kzz * v0sq + 2.f * szz - rho * v1sq +
-                    rho * v2sq) * (1.f / 24.f));
-    om = S.om_fix[4];
-    k[20] = om * (-(3.f * Kxx * v1 * v2 + 3.f * Kxxy * v2 + 3.f * Kxxyz + 3.f * Kxxz * v1 + 6.f * Kxy * v0 * v2 +
-                    6.f * Kxyz * v0 + 6.f * Kxz * v0 * v1 + 3.f * Kyz * v0sq - 2.f * Kyz - rho * v1 * v2) * (1.f / 24.f));
-    k[21] = om * (-(6.f * Kxy * v1 * v2 + 3.f * Kxyy * v2 + 3.f * Kxyyz + 6.f * Kxyz * v1 + 3.f * Kxz * v1sq -
-                    2.f * Kxz + 3.f * Kyy * v0 * v2 + 3.f * Kyyz * v0 + 6.f * Kyz * v0 * v1 - rho * v0 * v2) * (1.f / 24.f));
-    k[22] = om * (-(3.f * Kxy * v2sq - 2.f * Kxy + 6.f * Kxyz * v2 + 3.f * Kxyzz + 6.f * Kxz * v1 * v2 +
-                    3.f * Kxzz * v1 + 6.f * Kyz * v0 * v2 + 3.f * Kyzz * v0 + 3.f * Kzz * v0 * v1 - rho * v0 * v1) /
-                  24.f);
-    om = S.om_fix[5];
-    k[23] = om * (-(6.f * Kxy * v1 * v2sq - 4.f * Kxy * v1 + 3.f * Kxyy * v2sq - 2.f * Kxyy + 6.f * Kxyyz * v2 +
-                    3.f * Kxyyzz + 12.f * Kxyz * v1 * v2 + 6.f * Kxyzz * v1 + 6.f * Kxz * v1sq * v2 -
-                    4.f * Kxz * v2 + 3.f * Kxzz * v1sq - 2.f * Kxzz + 3.f * Kyy * v0 * v2sq - 2.f * Kyy * v0 +
-                    6.f * K[0][2][1] * v0 * v2 + 3.f * Kyyzz * v0 + 12.f * Kyz * v0 * v1 * v2 +
-                    6.f * Kyzz * v0 * v1 + 3.f * Kzz * v0 * v1sq - 2.f * Kzz * v0 - rho * v0 * v1sq -
-                    rho * v0 * v2sq + rho * v0) * (1.f / 24.f));
-    k[24] = om * (-(3.f * Kxx * v1 * v2sq - 2.f * Kxx * v1 + 3.f * Kxxy * v2sq - 2.f * Kxxy + 6.f * Kxxyz * v2 +
-                    3.f * Kxxyzz + 6.f * Kxxz * v1 * v2 + 3.f * Kxxzz * v1 + 6.f * Kxy * v0 * v2sq -
-                    4.f * Kxy * v0 + 12.f * Kxyz * v0 * v2 + 6.f * Kxyzz * v0 + 12.f * Kxz * v0 * v1 * v2 +
-                    6.f * Kxzz * v0 * v1 + 6.f * Kyz * v0sq * v2 - 4.f * Kyz * v2 + 3.f * Kyzz * v0sq -
-                    2.f * Kyzz + 3.f * Kzz * v0sq * v1 - 2.f * Kzz * v1 - rho * v0sq * v1 - rho * v1 * v2sq +
-                    rho * v1) * (1.f / 24.f));
-    k[25] = om * (-(3.f * Kxx * v1sq * v2 - 2.f * Kxx * v2 + 6.f * Kxxy * v1 * v2 + 3.f * Kxxyy * v2 +
-                    3.f * Kxxyyz + 6.f * Kxxyz * v1 + 3.f * Kxxz * v1sq - 2.f * Kxxz + 12.f * Kxy * v0 * v1 * v2 +
-                    6.f * Kxyy * v0 * v2 + 6.f * Kxyyz * v0 + 12.f * Kxyz * v0 * v1 + 6.f * Kxz * v0 * v1sq -
-                    4.f * Kxz * v0 + 3.f * Kyy * v0sq * v2 - 2.f * Kyy * v2 + 3.f * Kyyz * v0sq - 2.f * Kyyz +
-                    6.f * Kyz * v0sq * v1 - 4.f * Kyz * v1 - rho * v0sq * v2 - rho * v1sq * v2 + rho * v2) * (1.f / 24.f));
-    k[26] = om * (-(27.f * Kxx * v1sq * v2sq - 18.f * Kxx * v1sq - 18.f * Kxx * v2sq + 12.f * sxx +
-                    54.f * Kxxy * v1 * v2sq - 36.f * Kxxy * v1 + 27.f * Kxxyy * v2sq - 18.f * sxxyy +
-                    54.f * Kxxyyz * v2 + 27.f * sxxyyzz + 108.f * Kxxyz * v1 * v2 + 54.f * Kxxyzz * v1 +
-                    54.f * Kxxz * v1sq * v2 - 36.f * Kxxz * v2 + 27.f * Kxxzz * v1sq - 18.f * sxxzz +
-                    108.f * Kxy * v0 * v1 * v2sq - 72.f * Kxy * v0 * v1 + 54.f * Kxyy * v0 * v2sq -
-                    36.f * Kxyy * v0 + 108.f * Kxyyz * v0 * v2 + 54.f * Kxyyzz * v0 + 216.f * Kxyz * v0 * v1 * v2 +
-                    108.f * Kxyzz * v0 * v1 + 108.f * Kxz * v0 * v1sq * v2 - 72.f * Kxz * v0 * v2 +
-                    54.f * Kxzz * v0 * v1sq - 36.f * Kxzz * v0 + 27.f * Kyy * v0sq * v2sq - 18.f * Kyy * v0sq -
-                    18.f * Kyy * v2sq + 12.f * syy + 54.f * Kyyz * v0sq * v2 - 36.f * Kyyz * v2 +
-                    27.f * Kyyzz * v0sq - 18.f * syyzz + 108.f * Kyz * v0sq * v1 * v2 - 72.f * Kyz * v1 * v2 +
-                    54.f * Kyzz * v0sq * v1 - 36.f * Kyzz * v1 + 27.f * Kzz * v0sq * v1sq - 18.f * Kzz * v0sq -
-                    18.f * Kzz * v1sq + 12.f * szz - 9.f * rho * v0sq * v1sq - 9.f * rho * v0sq * v2sq +
-                    9.f * rho * v0sq - 9.f * rho * v1sq * v2sq + 9.f * rho * v1sq + 9.f * rho * v2sq -
-                    7.f * drho) * (1.f / 216.f));
-    // df = K k dt (detail/simulation_engine.cuh:518-527)
-#pragma unroll
-    for (int l = 0; l < 27; ++l) {
-        float s = 0.f;
-#pragma unroll
-        for (int j = 4; j < 27; ++j)
-            if (T::K(l, j) != 0) s += (float)T::K(l, j) * k[j];
-        delta[l] = s * S.dt_lat;
+        }
+    const float dt = S.dt_lat;
+    const float wa = -dt * S.om_ab, w0 = -dt * S.om_fix[0], w1 = -dt * S.om_fix[1], w2 = -dt * S.om_fix[2],
+                w3 = -dt * S.om_fix[3], w4 = -dt * S.om_fix[4], w5 = -dt * S.om_fix[5];
+    const float sxx = h[2][0][0], syy = h[0][2][0], szz = h[0][0][2], s2 = sxx + syy + szz;
+    const float sxy = h[2][2][0], sxz = h[2][0][2], syz = h[0][2][2], s4 = sxy + sxz + syz;
+    const float k7 = wa * (1.f / 12.f) * (sxx - syy);
+    const float k8 = wa * (1.f / 36.f) * (sxx + syy - 2.f * szz);
+    const float k9 = wa * (1.f / 18.f) * s2;
+    const float k17 = w3 * (1.f / 36.f) * (3.f * s4 - 4.f * s2);
+    const float k18 = w4 * (1.f / 72.f) * (3.f * (sxy + sxz - 2.f * syz) - 2.f * (2.f * sxx - syy - szz));
+    const float k19 = w4 * (1.f / 24.f) * (3.f * (sxy - sxz) - 2.f * (syy - szz));
+    const float k26 = w5 * (1.f / 216.f) * (27.f * h[2][2][2] - 18.f * s4 + 12.f * s2);
+    // even coefficients of the increment's polynomial in c
+    h[0][0][0] = -2.f * k9 + 4.f * k17 - 8.f * k26;
+    {
+        const float e = k9 - 4.f * k17 + 12.f * k26;
+        h[2][0][0] = e + k7 + k8 - 4.f * k18;
+        h[0][2][0] = e - k7 + k8 + 2.f * (k18 - k19);
+        h[0][0][2] = e - 2.f * k8 + 2.f * (k18 + k19);
+        const float q = 3.f * k17 - 18.f * k26;
+        h[2][2][0] = q + 3.f * (k18 + k19);
+        h[2][0][2] = q + 3.f * (k18 - k19);
+        h[0][2][2] = q - 6.f * k18;
+        h[2][2][2] = 27.f * k26;
     }
+    // the three pairs xy, xz, yz with their fourth-order partners
+    auto second = [&](float& ab, float& abcc) {
+        const float k = wa * (1.f / 12.f) * ab, kk = w4 * (1.f / 24.f) * (3.f * abcc - 2.f * ab);
+        ab = k - 2.f * kk;
+        abcc = 3.f * kk;
+    };
+    second(h[1][1][0], h[1][1][2]);
+    second(h[1][0][1], h[1][2][1]);
+    second(h[0][1][1], h[2][1][1]);
+    h[1][1][1] *= w2 * (1.f / 8.f);
+    // the axes: a b^2, a c^2 (third order) and a b^2 c^2 (fifth)
+    auto axis = [&](float& a, float& abb, float& acc, float& abbcc) {
+        const float t = abb + acc, k = w0 * (1.f / 72.f) * 3.f * t, kd = w1 * (1.f / 8.f) * (abb - acc);
+        const float kf = w5 * (1.f / 72.f) * (9.f * abbcc - 6.f * t);
+        a = 4.f * (kf - k);
+        const float e = 3.f * k - 6.f * kf;
+        abb = e + kd;
+        acc = e - kd;
+        abbcc = 9.f * kf;
+    };
+    axis(h[1][0][0], h[1][2][0], h[1][0][2], h[1][2][2]);
+    axis(h[0][1][0], h[2][1][0], h[0][1][2], h[2][1][2]);
+    axis(h[0][0][1], h[2][0][1], h[0][2][1], h[2][2][1]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) values(h[i][j][0], h[i][j][1], h[i][j][2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) values(h[i][0][j], h[i][1][j], h[i][2][j]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) values(h[0][i][j], h[1][i][j], h[2][i][j]);
+#pragma unroll
+    for (int a = 0; a < 27; ++a) delta[a] = h[T::cx(a) + 1][T::cy(a) + 1][T::cz(a) + 1];
 }
 
 // D2Q9 collision (detail/d2q9_lattice.cuh:120-299) with f = w + g. Terms
@@ -539,169 +462,6 @@ __device__ __forceinline__ void load_scene(SceneDev& dst, const SceneDev* src) {
         int* b = reinterpret_cast<int*>(&dst);
         for (int t = threadIdx.x; t < (int)(sizeof(SceneDev) / 4); t += 32) b[t] = a[t];
     }
-}
-
-#define NAGA_FOR_ITEMS(items, nitems)                           \
-    __shared__ SceneDev S;                                      \
-    pdl_wait_prev();                                            \
-    for (int w_ = blockIdx.x; w_ < (nitems); w_ += gridDim.x) { \
-        const WorkItem it = (items)[w_];                        \
-        __syncthreads();                                        \
-        load_scene(S, scenes + it.scene);                       \
-        __syncthreads();
-
-#define NAGA_END_ITEMS \
-    }                      \
-    pdl_allow_next();
-
-// Node-local part of the step, one thread per node (all nodes):
-// rho, u (stored for the probes and the next step); the PML trapezoid
-// integrals Q1 = (f~ + f~_prev) dt / 2, Q2 = (Q1 + Q1_prev) dt / 2 with
-// f~ = feq - w (pml_absorption.inl:531-631); the local absorption term
-// -sigma (3 f~ + 3 sigma Q1 + sigma^2 Q2) on layer nodes; the collision
-// increment K k dt (simulation_engine.cuh:469-531). Writes
-//   bulk/layer: S1 = g + local + collision, and S1P = g + local on nodes the
-//               boundary interpolation reads;
-//   boundary:   S1 = collision (the interpolated part is added later);
-//   ghost:      S1 = g + collision.
-// The item's rows of G and Q1_prev are staged in shared memory by coalesced
-// loads of the whole block before the (register-heavy) per-node work.
-// D3Q27 runs 4 blocks/SM (its collision needs the registers; tighter bounds
-// spill and were slower); D2Q9 fits 8 (one resident wave of the item grid;
-// at 7, 72 registers without spills, the 256-scene batch's kernel took 0.45
-// ms against 0.34)
-template <class L>
-__global__ void __launch_bounds__(kBlock, (L::D == 3 ? 4 : 8)) k_macro_pml(const WorkItem* __restrict__ items, int nitems,
-                                                         const SceneDev* __restrict__ scenes) {
-    constexpr int Q = L::Q, QP = L::QP;
-    // rows of the item's nodes: G and Q1_prev in, then the layer terms
-    // (Q1, Q2 of layer nodes, zero elsewhere) for the item's column sums
-    __shared__ float4 rowG[kBlock * QP / 4], rowQ[kBlock * QP / 4];
-    __shared__ double red[2][2 * QP];
-    NAGA_FOR_ITEMS(items, nitems)
-    const unsigned long long step = *S.step;
-    const int par = (int)(step & 1ull);
-    float* Q1cur = par ? S.Q1b : S.Q1a;
-    const float* Q1prev = par ? S.Q1a : S.Q1b;
-    const int nn = (int)(it.end - it.begin);
-    const int64_t i = (int64_t)it.begin + threadIdx.x;
-    const bool active = (int)threadIdx.x < nn;
-    const bool layer = active && i >= S.nb && i < S.nb + S.nl;
-    // node i carries NAGA's PML field of layer node i + pml_shift
-    const int64_t jf = i + S.pml_shift;
-    const bool field = active && jf >= S.nb && jf < S.nb + S.nl;
-    // per-node inputs issued before the row staging so their latency overlaps it
-    const float4 mp = active ? S.M[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float sg = layer ? __ldg(S.sigma + (i - S.nb)) : 0.f;
-    const float sf = field ? __ldg(S.sigma + (jf - S.nb)) : 0.f;
-    const bool src = active && i < S.nbl && S.is_src[i];
-    {
-        // copied with cp.async (16 B a thread and copy, no register staging),
-        // all of the thread's copies in flight at once
-        const float4* g4 = reinterpret_cast<const float4*>(S.G + (int64_t)it.begin * QP);
-        const float4* q4 = reinterpret_cast<const float4*>(Q1prev + (int64_t)it.begin * QP);
-        constexpr int NQ = QP / 4;  // float4 per row: the block moves kBlock * NQ of each
-        const int ne = nn * NQ;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int e = (int)threadIdx.x + q * kBlock;
-            if (e < ne) {
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(rowG + e)),
-                             "l"(g4 + e)
-                             : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(rowQ + e)),
-                             "l"(q4 + e)
-                             : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    float* myG = reinterpret_cast<float*>(rowG) + threadIdx.x * QP;
-    float* myQ = reinterpret_cast<float*>(rowQ) + threadIdx.x * QP;
-    if (active) {
-        float g[Q];
-#pragma unroll
-        for (int a = 0; a < Q; ++a) g[a] = myG[L::pos(a)];
-        float drho, u[3] = {0.f, 0.f, 0.f};
-        macros<L>(g, drho, u);
-        // density source of this step (after the probes sampled the macros):
-        // f_a += (s / rho0) w_a, and the reference's density statement
-        // rho <- (rho + (rho + s)) / 2 applied once, u unchanged
-        // (detail/simulation_engine.cuh:1057-1107 without its race)
-        if (S.src_slot) {
-            const int sl = S.src_slot[i];
-            const int64_t row = (int64_t)step - S.src_first;
-            if (sl >= 0 && row >= 0 && row < S.src_steps) {
-                const float sv = S.src_vals[row * S.src_n + sl];
-                if (sv != FLT_MAX) {
-                    const float ds = sv / S.rho0;
-#pragma unroll
-                    for (int a = 0; a < Q; ++a) g[a] = fmaf(ds, LatticeTables<L>::w(a), g[a]);
-                    drho += 0.5f * ds;
-                }
-            }
-        }
-        const float up[3] = {mp.y, mp.z, mp.w};
-        S.M[i] = make_float4(drho, u[0], u[1], L::D == 3 ? u[2] : 0.f);
-        float dcol[Q];
-        collide<L>(g, drho, u, S, dcol);
-        float q1[QP], out[QP], phi[QP];
-#pragma unroll
-        for (int t = 0; t < QP; ++t) q1[t] = out[t] = phi[t] = 0.f;
-#pragma unroll
-        for (int a = 0; a < Q; ++a) {
-            const int t = L::pos(a);
-            const float ft = feq_c<L>(a, drho, u);
-            const float ftp = feq_c<L>(a, mp.x, up);
-            q1[t] = (ft + ftp) * S.dt_lat / 2.f;
-            const float q2 = (q1[t] + myQ[t]) * S.dt_lat / 2.f;
-            phi[t] = -2.f * sf * q1[t] + sf * sf * q2;
-            myG[t] = layer ? q1[t] : 0.f;
-            myQ[t] = layer ? q2 : 0.f;
-            out[t] = layer ? g[a] - sg * (3.f * ft + 3.f * sg * q1[t] + sg * sg * q2) : g[a];
-        }
-        store_row<L>(Q1cur, i, q1);
-        if (field) {
-            // the field row holds the gathered chunks (L::QS floats)
-            float4* pr = reinterpret_cast<float4*>(S.PHI + (jf - S.nb) * L::QS);
-#pragma unroll
-            for (int c = 0; c < L::QS / 4; ++c)
-                pr[c] = make_float4(phi[4 * c], phi[4 * c + 1], phi[4 * c + 2], phi[4 * c + 3]);
-        }
-        if (src) s1_store_row<L>(S.S1P, S.N, i, out);
-        const bool boundary = i >= S.nbl && i < S.nbl + S.nbd;
-#pragma unroll
-        for (int a = 0; a < Q; ++a) {
-            const int t = L::pos(a);
-            out[t] = boundary ? dcol[a] : out[t] + dcol[a];
-        }
-        s1_store_row<L>(S.S1, S.N, i, out);
-    } else {
-#pragma unroll
-        for (int t = 0; t < QP; ++t) myG[t] = myQ[t] = 0.f;
-    }
-    // per-item layer sums of Q1 and Q2 in FP64, fixed order: column t of
-    // the rows, two halves of the item summed in node order, then added
-    const bool touches = (int64_t)it.end > S.nb && (int64_t)it.begin < S.nb + S.nl;
-    __syncthreads();
-    if (touches && threadIdx.x < 4 * QP) {
-        const int col = threadIdx.x % (2 * QP), half = threadIdx.x / (2 * QP);
-        const float* base = col < QP ? reinterpret_cast<const float*>(rowG) : reinterpret_cast<const float*>(rowQ);
-        const int t = col < QP ? col : col - QP;
-        const int r0 = half * (kBlock / 2), r1 = min(nn, r0 + kBlock / 2);
-        double v = 0.0;
-        for (int r = r0; r < r1; ++r) v += (double)base[r * QP + t];
-        red[half][col] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 2 * QP)
-        S.partials[(int64_t)threadIdx.x * S.n_all_items + it.local] =
-            touches ? red[0][threadIdx.x] + red[1][threadIdx.x] : 0.0;
-    NAGA_END_ITEMS
 }
 
 // Per-scene tail of the node-local pass, one launch for all scenes:
@@ -807,6 +567,30 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
+// two such copies of the same size on one phase
+__device__ __forceinline__ void bulk_load2(void* dst0, const void* src0, void* dst1, const void* src1, uint32_t bytes,
+                                           uint64_t* bar) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(2 * bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst0)),
+                 "l"(src0), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst1)),
+                 "l"(src1), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+// one bulk copy shared -> global in the thread's current bulk group (the
+// writers of the shared memory fenced it for the async proxy)
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
+                 "r"(bytes)
+                 : "memory");
+}
+
 // bounded wait for the phase of `bar` with the given parity; false if the
 // copy did not complete within `polls` polls. A failed poll suspends the
 // thread for a hardware-defined time (about 4 us measured on B200 when
@@ -839,6 +623,207 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __device__ unsigned int g_tile_timeout;
 
 namespace {
+
+// Node-local part of the step, one thread per node (all nodes):
+// rho, u (stored for the probes and the next step); the PML trapezoid
+// integrals Q1 = (f~ + f~_prev) dt / 2, Q2 = (Q1 + Q1_prev) dt / 2 with
+// f~ = feq - w (pml_absorption.inl:531-631); the local absorption term
+// -sigma (3 f~ + 3 sigma Q1 + sigma^2 Q2) on layer nodes; the collision
+// increment K k dt (simulation_engine.cuh:469-531). Writes
+//   bulk/layer: S1 = g + local + collision, and S1P = g + local on nodes the
+//               boundary interpolation reads;
+//   boundary:   S1 = collision (the interpolated part is added later);
+//   ghost:      S1 = g + collision.
+// An item's rows are contiguous, so G and Q1_prev come into shared memory and
+// S1 and Q1 leave it as one bulk copy each (a thread storing its own 112-B
+// row touches 32 lines per warp-wide store). A thread reads and rewrites its
+// row four populations at a time (16-B accesses at the odd stride of 7 float4:
+// no bank conflicts), and reads g again after the collision instead of
+// keeping it in registers through it. Against per-thread row stores and the
+// collision in central moments: D3Q27 250k nodes 48 -> 33 us, 1M nodes 170 ->
+// 109 us (0.62 of the copy bandwidth over its compulsory bytes); 32 ragged
+// D2Q9 scenes, 0.95 M nodes, 53 -> 47 us. What is left above HBM is the
+// latency of the two row copies at the head of an item and the field rows'
+// stores.
+// D3Q27 runs 4 blocks/SM (its collision needs the registers); D2Q9 fits 8 (one
+// resident wave of the item grid; at 7, 72 registers without spills, the
+// 256-scene batch's kernel took 0.45 ms against 0.34)
+template <class L>
+__global__ void __launch_bounds__(kBlock, (L::D == 3 ? 4 : 8)) k_macro_pml(const WorkItem* __restrict__ items, int nitems,
+                                                         const SceneDev* __restrict__ scenes) {
+    constexpr int Q = L::Q, QP = L::QP, NQ = QP / 4;
+    // S1 rows: D3Q27 full rows, built in place of G; D2Q9 the pairs (s1_ld),
+    // in a buffer of their own (another stride than G's rows)
+    constexpr int NS = L::D == 3 ? NQ : L::NGATHER;
+    __shared__ __align__(128) float4 rowG[kBlock * NQ], rowQ[kBlock * NQ], rowQ2[kBlock * NQ];
+    __shared__ __align__(128) float4 rowS_[L::D == 3 ? 1 : kBlock * NS];
+    float4* const rowS = L::D == 3 ? rowG : rowS_;
+    __shared__ double red[2][2 * QP];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ SceneDev S;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar);
+        mbar_init_fence();
+    }
+    uint32_t phase = 0;
+    WorkItem it = (int)blockIdx.x < nitems ? items[blockIdx.x] : WorkItem{0u, 0u, 0u, 0u};
+    if ((int)blockIdx.x < nitems) load_scene(S, scenes + it.scene);
+    __syncthreads();
+    pdl_wait_prev();
+    for (int w_ = blockIdx.x; w_ < nitems;) {
+        const unsigned long long step = *S.step;
+        const int par = (int)(step & 1ull);
+        float* const Q1cur = par ? S.Q1b : S.Q1a;
+        const float* const Q1prev = par ? S.Q1a : S.Q1b;
+        const int nn = (int)(it.end - it.begin);
+        const uint32_t row_bytes = (uint32_t)(nn * QP * sizeof(float));
+        if (threadIdx.x == 0)
+            bulk_load2(rowG, S.G + (int64_t)it.begin * QP, rowQ, Q1prev + (int64_t)it.begin * QP, row_bytes, &bar);
+        const int64_t i = (int64_t)it.begin + threadIdx.x;
+        const bool active = (int)threadIdx.x < nn;
+        const bool layer = active && i >= S.nb && i < S.nb + S.nl;
+        // node i carries NAGA's PML field of layer node i + pml_shift
+        const int64_t jf = i + S.pml_shift;
+        const bool field = active && jf >= S.nb && jf < S.nb + S.nl;
+        // per-node inputs issued before the wait for the rows
+        const float4 mp = active ? S.M[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float sg = layer ? __ldg(S.sigma + (i - S.nb)) : 0.f;
+        const float sf = field ? __ldg(S.sigma + (jf - S.nb)) : 0.f;
+        const bool src = active && i < S.nbl && S.is_src[i];
+        // rows of the item inside the layer
+        const int l0 = (int)max((int64_t)0, S.nb - (int64_t)it.begin);
+        const int l1 = (int)min((int64_t)nn, S.nb + S.nl - (int64_t)it.begin);
+        const bool touches = l0 < l1;
+        const bool ok = mbar_wait(&bar, phase);
+        phase ^= 1u;
+        if (__syncthreads_or(!ok)) {
+            if (threadIdx.x == 0) {
+                atomicOr(&g_tile_timeout, 1u);
+                if (!ok) mbar_wait(&bar, phase ^ 1u);  // the copies still in flight
+            }
+            return;
+        }
+        float4* const myG = rowG + threadIdx.x * NQ;
+        float4* const myQ = rowQ + threadIdx.x * NQ;
+        if (active) {
+            float drho, u[3] = {0.f, 0.f, 0.f};
+            float dcol[Q];
+            {
+                float g[Q];
+#pragma unroll
+                for (int c = 0; c < NQ; ++c) {
+                    const float4 v = myG[c];
+                    if (L::row(4 * c) >= 0) g[L::row(4 * c)] = v.x;
+                    if (L::row(4 * c + 1) >= 0) g[L::row(4 * c + 1)] = v.y;
+                    if (L::row(4 * c + 2) >= 0) g[L::row(4 * c + 2)] = v.z;
+                    if (L::row(4 * c + 3) >= 0) g[L::row(4 * c + 3)] = v.w;
+                }
+                macros<L>(g, drho, u);
+                // density source of this step (after the probes sampled the
+                // macros): f_a += (s / rho0) w_a, and the reference's density
+                // statement rho <- (rho + (rho + s)) / 2 applied once, u
+                // unchanged (detail/simulation_engine.cuh:1057-1107 without
+                // its race)
+                if (S.src_slot) {
+                    const int sl = S.src_slot[i];
+                    const int64_t row = (int64_t)step - S.src_first;
+                    if (sl >= 0 && row >= 0 && row < S.src_steps) {
+                        const float sv = S.src_vals[row * S.src_n + sl];
+                        if (sv != FLT_MAX) {
+                            const float ds = sv / S.rho0;
+                            float* const gs = reinterpret_cast<float*>(myG);
+#pragma unroll
+                            for (int a = 0; a < Q; ++a) {
+                                g[a] = fmaf(ds, LatticeTables<L>::w(a), g[a]);
+                                gs[L::pos(a)] = g[a];
+                            }
+                            drho += 0.5f * ds;
+                        }
+                    }
+                }
+                S.M[i] = make_float4(drho, u[0], u[1], L::D == 3 ? u[2] : 0.f);
+                collide<L>(g, drho, u, S, dcol);
+            }
+            const float up[3] = {mp.y, mp.z, mp.w};
+            const float hdt = S.dt_lat / 2.f;
+            const float uu = u[0] * u[0] + u[1] * u[1] + (L::D == 3 ? u[2] * u[2] : 0.f);
+            const float uup = up[0] * up[0] + up[1] * up[1] + (L::D == 3 ? up[2] * up[2] : 0.f);
+            const bool boundary = i >= S.nbl && i < S.nbl + S.nbd;
+            float4* const pr = reinterpret_cast<float4*>(S.PHI + (jf - S.nb) * L::QS);
+#pragma unroll
+            for (int c = 0; c < NQ; ++c) {
+                const float4 g4 = myG[c], p4 = myQ[c];
+                const float gv[4] = {g4.x, g4.y, g4.z, g4.w}, pv[4] = {p4.x, p4.y, p4.z, p4.w};
+                float q1[4], q2[4], phi[4], out[4], s1[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    // slots 4c + 2h, 4c + 2h + 1: a direction and its
+                    // opposite, or the rest population and a pad
+                    float ft[2], fp[2];
+                    feq_pair<L>(L::row(4 * c + 2 * h), drho, u, uu, ft);
+                    feq_pair<L>(L::row(4 * c + 2 * h), mp.x, up, uup, fp);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int t = 2 * h + e, a = L::row(4 * c + t);
+                        if (a < 0) {
+                            q1[t] = q2[t] = phi[t] = out[t] = s1[t] = 0.f;
+                            continue;
+                        }
+                        q1[t] = (ft[e] + fp[e]) * hdt;
+                        q2[t] = (q1[t] + pv[t]) * hdt;
+                        phi[t] = sf * (sf * q2[t] - 2.f * q1[t]);
+                        out[t] = gv[t] - sg * (3.f * ft[e] + sg * (3.f * q1[t] + sg * q2[t]));
+                        s1[t] = boundary ? dcol[a] : out[t] + dcol[a];
+                    }
+                }
+                myQ[c] = make_float4(q1[0], q1[1], q1[2], q1[3]);
+                if (touches) rowQ2[threadIdx.x * NQ + c] = make_float4(q2[0], q2[1], q2[2], q2[3]);
+                // the field row holds the gathered chunks (L::QS floats)
+                if (field && c < L::QS / 4) pr[c] = make_float4(phi[0], phi[1], phi[2], phi[3]);
+                if (src) s1_st<L>(S.S1P, S.N, i, c, make_float4(out[0], out[1], out[2], out[3]));
+                if (c < NS)
+                    rowS[threadIdx.x * NS + c] = make_float4(s1[0], s1[1], s1[2], s1[3]);
+                else
+                    s1_st<L>(S.S1, S.N, i, c, make_float4(s1[0], s1[1], s1[2], s1[3]));
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            bulk_store(Q1cur + (int64_t)it.begin * QP, rowQ, row_bytes);
+            bulk_store(S.S1 + (int64_t)it.begin * (4 * NS), rowS, (uint32_t)(nn * NS * sizeof(float4)));
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        // per-item layer sums of Q1 and Q2 in FP64, fixed order: column t of
+        // the layer's rows, two halves of the item summed in node order, then
+        // added
+        if (touches && threadIdx.x < 4 * QP) {
+            const int col = threadIdx.x % (2 * QP), half = threadIdx.x / (2 * QP);
+            const float* base = reinterpret_cast<const float*>(col < QP ? rowQ : rowQ2);
+            const int t = col < QP ? col : col - QP;
+            const int r0 = max(half * (kBlock / 2), l0), r1 = min((half + 1) * (kBlock / 2), l1);
+            double v = 0.0;
+            for (int r = r0; r < r1; ++r) v += (double)base[r * QP + t];
+            red[half][col] = v;
+        }
+        const int local = (int)it.local;
+        const int w_next = w_ + (int)gridDim.x;
+        if (w_next < nitems) it = items[w_next];
+        __syncthreads();
+        if (threadIdx.x < 2 * QP)
+            S.partials[(int64_t)threadIdx.x * S.n_all_items + local] =
+                touches ? red[0][threadIdx.x] + red[1][threadIdx.x] : 0.0;
+        w_ = w_next;
+        if (w_ >= nitems) break;
+        // the stores have read the rows before the next item's copies land
+        if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncthreads();
+        load_scene(S, scenes + it.scene);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    pdl_allow_next();
+}
 
 template <class T>
 __device__ __forceinline__ void copy_tile(T* tile, TileSrc src) {
