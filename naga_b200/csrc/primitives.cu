@@ -23,9 +23,9 @@
 
 namespace naga {
 
-int rbf_weights_device(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const double* qry,
-                       int64_t ngroups, int group, double spacing, int shape, int precision, double* weights,
-                       cudaStream_t st);
+int rbf_weights_f32_device(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const float* qry,
+                           int64_t ngroups, int group, double spacing, int shape, int precision, float* weights,
+                           cudaStream_t st);
 
 namespace {
 
@@ -135,16 +135,7 @@ int seg_grid_from_bounds(int dim, int64_t n, int approx, const int* hb, SegGrid&
     return NAGA_OK;
 }
 
-// ---------------------------------------------------------- RPIM, FP32 I/O
-__global__ void widen_kernel(const float* __restrict__ in, double* __restrict__ out, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (double)in[i];
-}
-__global__ void narrow_kernel(const double* __restrict__ in, float* __restrict__ out, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (float)in[i];
-}
-
+// ------------------------------------------------------ RPIM interpolation
 // destination(c, q) = sum_s w(s, q) (field(c, support(s, q / group)) - offset)
 // + offset, summed over s in order in FP32 (radial_point_method.cuh:204-218,
 // 243-257); one thread per (component, query)
@@ -310,23 +301,8 @@ extern "C" int naga_rbf_weights_f32(const float* src, int64_t n, int dim, const 
     if (dim != 2 && dim != 3) return set_error(NAGA_EINVAL, "naga_rbf_weights_f32: dim must be 2 or 3");
     if (k < 1 || k > 64) return set_error(NAGA_EINVAL, "naga_rbf_weights_f32: k out of range");
     cudaStream_t st = (cudaStream_t)stream;
-    const int64_t nq = ngroups * group;
-    double *q64 = nullptr, *w64 = nullptr;
-    NAGA_CUDA_TRY(scratch_malloc(&q64, sizeof(double) * nq * dim, st));
-    NAGA_CUDA_TRY(scratch_malloc(&w64, sizeof(double) * nq * k, st));
-    const int b1 = (int)std::min<int64_t>((nq * dim + 255) / 256, (int64_t)sm_count() * 8);
-    widen_kernel<<<b1, 256, 0, st>>>(qry, q64, nq * dim);
-    NAGA_CUDA_TRY(cudaGetLastError());
-    int rc = rbf_weights_device(src, n, dim, support, k, q64, ngroups, group, (double)spacing, shape, precision,
-                                w64, st);
-    if (rc == NAGA_OK) {
-        const int b2 = (int)std::min<int64_t>((nq * k + 255) / 256, (int64_t)sm_count() * 8);
-        narrow_kernel<<<b2, 256, 0, st>>>(w64, weights, nq * k);
-        if (cudaGetLastError() != cudaSuccess) rc = set_error(NAGA_ECUDA, "naga_rbf_weights_f32: narrow kernel");
-    }
-    cudaFreeAsync(q64, st);
-    cudaFreeAsync(w64, st);
-    return rc;
+    return rbf_weights_f32_device(src, n, dim, support, k, qry, ngroups, group, (double)spacing, shape, precision,
+                                  weights, st);
 }
 
 extern "C" int naga_rbf_interpolate(const float* weights, const uint32_t* support, int64_t nq, int group, int k,

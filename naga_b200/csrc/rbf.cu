@@ -14,12 +14,14 @@
 // block scales by a constant and span{1, x} is shift- and scale-invariant)
 // while it removes most of the ill-conditioning of the absolute-coordinate
 // system.
+#include "warp_gj.cuh"
 #include "warp_lu.cuh"
 #include "scene_dev.hpp"
 #include "scratch.hpp"
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace naga {
@@ -283,9 +285,12 @@ __device__ __forceinline__ void kernel_and_weight(double delta, const double* xy
 struct QuadTable {
     double u[64][3];
     double K[64][3];
-    double ksum[3];  // sum_q K_qd
+    double ksum[3];   // sum_q K_qd
+    double mom[3][3];  // sum_q K_qd u_qe: [d][e]
+    double len2[4];    // |u_q|^2 of the four radii
 };
-__device__ QuadTable g_quad[2];  // D2Q9, D3Q27 (filled once per device)
+__device__ QuadTable g_quad[2];    // D2Q9, D3Q27 (filled once per device)
+__constant__ QuadTable c_quad[2];  // copy of g_quad for the warp-uniform reads of quad_row
 
 template <int D>
 __global__ void quad_table_kernel() {
@@ -302,11 +307,20 @@ __global__ void quad_table_kernel() {
             g_q.K[q][d] = d < D ? a[d] * wq : 0.0;
         }
     }
+    if (q < 4) {
+        const double r = (c_gl_x[q] + 1.0) / 2.0;
+        g_q.len2[q] = r * r;
+    }
     __syncthreads();
     if (q < 3) {
         double sum = 0;
         for (int t = 0; t < nq; ++t) sum += g_q.K[t][q];  // fixed order
         g_q.ksum[q] = sum;
+        for (int e = 0; e < 3; ++e) {
+            sum = 0;
+            for (int t = 0; t < nq; ++t) sum += g_q.K[t][q] * g_q.u[t][e];
+            g_q.mom[q][e] = sum;
+        }
     }
 }
 
@@ -536,244 +550,256 @@ __global__ void divergence_build_kernel(const float* __restrict__ pts, int64_t n
     }
 }
 
-// ---- fixed stencil size, FP64: the augmented system [G0 | b_1 .. b_D] is
-// factored in place, row-major with a padded row stride, so the forward
-// substitution rides along with the elimination and one back substitution
-// serves the D right-hand sides. Pivoting is warp_lu's (first maximal |a|
-// of the column, rows swapped whole), the updates are the same operations
-// in the same order; the back substitution multiplies by the pivot's
-// reciprocal (computed once per column) instead of dividing.
-template <int D, int KC>
-struct AugSize {
-    static constexpr int N = KC + D + 1;              // system size
-    static constexpr int NC = (N + D + 1) / 2 * 2;    // columns with the right-hand sides, even
-    static constexpr int LD = NC % 4 == 2 ? NC : NC + 2;  // row stride: 16-B rows, lanes' rows on distinct banks
-    static constexpr int OFF = N > 32 ? N - 32 : 0;   // lane l owns row OFF + l, lanes < OFF also row l
-    // per-warp block, a multiple of 128 B so every warp's rows stay 16-B aligned
-    static constexpr size_t smem_per_warp = (sizeof(double) * ((size_t)N * LD + (size_t)KC * D + N) + 127) / 128 * 128;
-};
-static_assert(AugSize<3, 32>::LD % 2 == 0 && AugSize<2, 16>::LD % 2 == 0, "16-B aligned rows");
-static_assert(AugSize<3, 32>::smem_per_warp % 16 == 0 && AugSize<2, 16>::smem_per_warp % 16 == 0, "aligned warps");
+// ---- stencils of up to 32 supports in FP64: the register Gauss-Jordan solve
+// of warp_gj.cuh. KC is the stencil size rounded up (16, 24, 32); the rows and
+// columns past k are those of the identity.
 
-// G0 row-major with stride LD (G0 is symmetric, so this is also its transpose)
-template <int D, int KC>
-__device__ __forceinline__ void build_G0_rows(const double* xs, int shape, double* A) {
-    using Z = AugSize<D, KC>;
-    if constexpr (KC == 32) {
-        // RBF block by symmetry: lane l evaluates the pairs (l, l + t mod 32),
-        // t = 0..16, and writes both mirror entries (the t = 16 pairs twice,
-        // with the same value)
-        const int l = lane_id();
-        double xl[D];
+// The support rows of the moment matrix into sys.a (right-hand sides not
+// touched) from the scaled support coordinates xs. The RBF block by symmetry:
+// lane l evaluates the pairs (l, l + t mod KC), t = 0 .. KC / 2, and writes
+// both mirror entries to the assembly rows, of which it then reads its own.
+template <int D, int KC, int NR>
+__device__ __forceinline__ void assemble(GjSystem<KC, D, NR>& sys, const double* xs, int k, int shape, double* rows) {
+    using S = GjSystem<KC, D, NR>;
+    const int l = lane_id();
+    double xl[D];
 #pragma unroll
-        for (int d = 0; d < D; ++d) xl[d] = xs[l * D + d];
-#pragma unroll 4
-        for (int t = 0; t <= 16; ++t) {
-            const int c = (l + t) & 31;
+    for (int d = 0; d < D; ++d) xl[d] = l < k ? xs[l * D + d] : 0.0;
+    if (l < KC) {
+#pragma unroll 3
+        for (int t = 0; t <= KC / 2; ++t) {
+            const int c = l + t < KC ? l + t : l + t - KC;
             double r2 = 0;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-                const double u = xl[d] - xs[c * D + d];
+                const double u = xl[d] - (c < k ? xs[c * D + d] : 0.0);
                 r2 += u * u;
             }
-            const double v = shape_fn(r2, shape);
-            A[l * Z::LD + c] = v;
-            A[c * Z::LD + l] = v;
+            const double v = l < k && c < k ? shape_fn(r2, shape) : (l == c ? 1.0 : 0.0);
+            rows[l * S::LD + c] = v;
+            rows[c * S::LD + l] = v;
         }
-        // border [1, x] in row / column l, and the zero corner
-        A[l * Z::LD + KC] = 1.0;
-        A[KC * Z::LD + l] = 1.0;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            A[l * Z::LD + KC + 1 + d] = xl[d];
-            A[(KC + 1 + d) * Z::LD + l] = xl[d];
-        }
-        if (l < (D + 1) * (D + 1)) A[(KC + l / (D + 1)) * Z::LD + KC + l % (D + 1)] = 0.0;
-        return;
     }
-#pragma unroll 4
-    for (int e = lane_id(); e < Z::N * Z::N; e += 32) {
-        const int r = e / Z::N, c = e % Z::N;
-        double v;
-        if (r >= KC && c >= KC)
-            v = 0.0;
-        else if (r >= KC)
-            v = (r == KC) ? 1.0 : xs[c * D + (r - KC - 1)];
-        else if (c >= KC)
-            v = (c == KC) ? 1.0 : xs[r * D + (c - KC - 1)];
-        else {
-            double r2 = 0;
+    __syncwarp();
+    const double* row = rows + (l < KC ? l : 0) * S::LD;
+    sys.a[0] = l < k ? 1.0 : 0.0;
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-                const double t = xs[r * D + d] - xs[c * D + d];
-                r2 += t * t;
-            }
-            v = shape_fn(r2, shape);
-        }
-        A[r * Z::LD + c] = v;
+    for (int d = 0; d < D; ++d) sys.a[1 + d] = xl[d];
+#pragma unroll
+    for (int m = 0; m < KC; m += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(row + m);
+        sys.a[S::E + m] = v.x;
+        sys.a[S::E + m + 1] = v.y;
     }
+#pragma unroll
+    for (int m = S::E + KC + NR; m < S::W; ++m) sys.a[m] = 0.0;
+    __syncwarp();  // the rows are read: solve() puts the solution there
 }
 
-// row i -= l_i * row j over columns j+1 .. NC-1, l_i = a_ij / a_jj stored
-template <int NC>
-__device__ __forceinline__ void eliminate_row(double* ri, const double* rj, int j, double inv) {
-    const double l = ri[j] * inv;
-    ri[j] = l;
-    int c = j + 1;
-    if (c & 1) {
-        ri[c] -= l * rj[c];
-        ++c;
+// Right-hand side of support row lane: b_d = sum_q alpha_d(q) w_q phi(|x - x_q|)
+// from the delta = 1 table (x_q = delta u_q / h, alpha_d w_q = K_qd / delta).
+// The four angles theta of a radius and polar angle are (+-s, 0), (0, +-s) with
+// one s, z and one kernel value each way, so they share their part of |x -
+// x_q|^2 and enter b as differences and one sum.
+template <int D>
+__device__ __forceinline__ void quad_row(const double* xl, int shape, double us, double rdel, double* b) {
+    const QuadTable& tq = c_quad[D - 2];
+    double x2 = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        b[d] = 0;
+        x2 = fma(xl[d], xl[d], x2);
     }
-    for (; c < NC; c += 2) {
-        double2 a = *reinterpret_cast<double2*>(ri + c);
-        const double2 b = *reinterpret_cast<const double2*>(rj + c);
-        a.x -= l * b.x;
-        a.y -= l * b.y;
-        *reinterpret_cast<double2*>(ri + c) = a;
-    }
+    const double us2 = us * us, m0 = -2.0 * us * xl[0], m1 = -2.0 * us * xl[1], m2 = D == 3 ? -2.0 * us * xl[D - 1] : 0.0;
+#pragma unroll 1
+    for (int p = 0; p < (D == 2 ? 1 : 4); ++p)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int q = 16 * p + r;  // theta = 0
+            const double s = tq.u[q][0], z = tq.u[q][2];
+            double base = fma(us2, tq.len2[r], x2);
+            if (D == 3) base = fma(m2, z, base);
+            // |x - x_q|^2 >= 0: the expanded form may round below for a
+            // support at the node
+            const double g0 = shape_fn(fmax(fma(m0, s, base), 0.0), shape);
+            const double g2 = shape_fn(fmax(fma(-m0, s, base), 0.0), shape);
+            const double g1 = shape_fn(fmax(fma(m1, s, base), 0.0), shape);
+            const double g3 = shape_fn(fmax(fma(-m1, s, base), 0.0), shape);
+            const double ks = tq.K[q][0];
+            b[0] = fma(ks, g0 - g2, b[0]);
+            b[1] = fma(ks, g1 - g3, b[1]);
+            if (D == 3) b[D - 1] = fma(tq.K[q][2], (g0 + g2) + (g1 + g3), b[D - 1]);
+        }
+#pragma unroll
+    for (int d = 0; d < D; ++d) b[d] *= rdel;
 }
 
-// In-place LU of the augmented rows; rdiag[j] = 1 / u_jj. Returns 0, or
-// j + 1 for the first column whose pivot is exactly zero (left unreduced).
+constexpr int kGjBlockWarps = 4;
+
+// Measured against the LU in shared memory that it replaces (every
+// multiply-add a shared-memory read-modify-write, 9 wavefronts per two columns
+// of a row): 250k nodes, k = 32: 8.6 -> 2.9 ms (100k nodes 3.7 -> 1.2 ms);
+// 50k weights 1.70 -> 0.45 ms. Bound by instruction issue at 16 warps/SM (128
+// registers): half the issue slots, the FP64 pipe 28 % (the square roots of the
+// quadrature and the elimination in about equal parts). Relative error of the
+// FP64 weights against another FP64 solve: 1.1e-13, the LU 0.9e-13.
 template <int D, int KC>
-__device__ int aug_lu(double* A, double* rdiag) {
-    using Z = AugSize<D, KC>;
-    constexpr int N = Z::N, LD = Z::LD, OFF = Z::OFF;
-    const int lane = lane_id();
-    const int p1 = OFF + lane;
-    const bool has1 = p1 < N, has2 = lane < OFF;
-    int info = 0;
-    for (int j = 0; j < N; ++j) {
-        // NaN never becomes a candidate, so the comparisons order totally and
-        // every lane ends with the same pivot; lane 0's is broadcast anyway,
-        // and a column with no candidate (all NaN) pivots on its own row
-        double best = -1.0;
-        int bi = N;
-        if (has2 && lane >= j) {
-            const double v = fabs(A[lane * LD + j]);
-            if (v > best) {
-                best = v;
-                bi = lane;
-            }
-        }
-        if (has1 && p1 >= j) {
-            const double v = fabs(A[p1 * LD + j]);
-            if (v > best) {
-                best = v;
-                bi = p1;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(kFull, best, o);
-            const int oi = __shfl_xor_sync(kFull, bi, o);
-            if (ov > best || (ov == best && oi < bi)) {
-                best = ov;
-                bi = oi;
-            }
-        }
-        bi = __shfl_sync(kFull, bi, 0);
-        const int p = bi < N ? bi : j;
-        if (A[p * LD + j] == 0.0) {
-            if (!info) info = j + 1;
-            if (lane == 0) rdiag[j] = 0.0;
-            __syncwarp();
-            continue;
-        }
-        if (p != j)
-            for (int c = lane; c < Z::NC; c += 32) {
-                const double t = A[j * LD + c];
-                A[j * LD + c] = A[p * LD + c];
-                A[p * LD + c] = t;
-            }
-        __syncwarp();
-        const double inv = 1.0 / A[j * LD + j];
-        if (lane == 0) rdiag[j] = inv;
-        if (has1 && p1 > j) eliminate_row<Z::NC>(A + p1 * LD, A + j * LD, j, inv);
-        if (has2 && lane > j) eliminate_row<Z::NC>(A + lane * LD, A + j * LD, j, inv);
-        __syncwarp();
-    }
-    return info;
-}
-
-template <int D, int KC>
-__global__ void divergence_build_fixed_kernel(const float* __restrict__ pts, int64_t n,
-                                              const uint32_t* __restrict__ idx, const double* __restrict__ spacing,
-                                              int64_t spacing_batch, int shape, StencilOut out,
-                                              int* __restrict__ status, int wpb) {
-    using Z = AugSize<D, KC>;
-    constexpr int N = Z::N, LD = Z::LD, OFF = Z::OFF;
-    static_assert(KC <= 32, "one support per lane");
+__global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
+    divergence_build_gj_kernel(const float* __restrict__ pts, int64_t n, const uint32_t* __restrict__ idx, int k,
+                               const double* __restrict__ spacing, int64_t spacing_batch, int shape, StencilOut out,
+                               int* __restrict__ status) {
+    using S = GjSystem<KC, D, D>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = lane_id();
-    double* A = reinterpret_cast<double*>(smem + Z::smem_per_warp * w);
-    double* xs = A + N * LD;
-    double* rdiag = xs + KC * D;
-    const int p1 = OFF + lane;
-    const bool has1 = p1 < N, has2 = lane < OFF;
-    for (int64_t i = (int64_t)blockIdx.x * wpb + w; i < n; i += (int64_t)gridDim.x * wpb) {
-        const NodeStencil<D> ns = load_node<D>(pts, n, idx, KC, i, spacing[i / spacing_batch], xs);
+    double* rows = reinterpret_cast<double*>(smem) + (size_t)S::doubles * w;
+    double* pr = rows + S::kAsm;
+    double* rhs = pr + S::kRow;
+    double* xs = rhs + S::kRhs;
+    for (int64_t i = (int64_t)blockIdx.x * kGjBlockWarps + w; i < n; i += (int64_t)gridDim.x * kGjBlockWarps) {
+        const NodeStencil<D> ns = load_node<D>(pts, n, idx, k, i, spacing[i / spacing_batch], xs);
         if (ns.bad && lane == 0) atomicOr(status, 1);
-        build_G0_rows<D, KC>(xs, shape, A);
-        double b0[D], b1[D], cself[D];
-        quad_rhs<D>(xs, KC, N, shape, ns, b0, b1, cself);
-        // right-hand-side columns N .. N+D-1 (original row order), zero padding
-        for (int r = 0; r < 2; ++r) {
-            const int row = lane + 32 * r;
-            if (row < N) {
+        const double rdel = 1.0 / ns.delta, us = ns.delta / ns.sp;
+        const QuadTable& tq = c_quad[D - 2];
+        double xl[D], b[D];
 #pragma unroll
-                for (int d = 0; d < D; ++d) A[row * LD + N + d] = r == 0 ? b0[d] : b1[d];
-                for (int c = N + D; c < Z::NC; ++c) A[row * LD + c] = 0.0;
-            }
+        for (int d = 0; d < D; ++d) xl[d] = lane < k ? xs[lane * D + d] : 0.0;
+        quad_row<D>(xl, shape, us, rdel, b);
+        S sys;
+        assemble<D, KC, D>(sys, xs, k, shape, rows);
+#pragma unroll
+        for (int d = 0; d < D; ++d) sys.a[S::E + KC + d] = lane < k ? b[d] : 0.0;
+        // the constraints' right-hand sides: sum_q alpha_d w_q (1, x_q)
+        if (lane < S::kRhs) {
+            const int r = lane / D, d = lane % D;
+            rhs[lane] = r == 0 ? tq.ksum[d] * rdel : tq.mom[d][r - 1] * us * rdel;
         }
         __syncwarp();
-        if (aug_lu<D, KC>(A, rdiag)) atomicOr(status, 2);
-        // back substitution, all right-hand sides at once: y1 holds row
-        // OFF + lane, y2 row lane (lanes < OFF)
-        double y1[D], y2[D];
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            y1[d] = has1 ? A[p1 * LD + N + d] : 0.0;
-            y2[d] = has2 ? A[lane * LD + N + d] : 0.0;
-        }
-        for (int j = N - 1; j >= 0; --j) {
-            const double rj = rdiag[j];
-            double xj[D];
-#pragma unroll
-            for (int d = 0; d < D; ++d)
-                xj[d] = (j >= OFF ? __shfl_sync(kFull, y1[d], j - OFF) : __shfl_sync(kFull, y2[d], j)) * rj;
-            if (has1) {
-                if (p1 == j) {
-#pragma unroll
-                    for (int d = 0; d < D; ++d) y1[d] = xj[d];
-                } else if (p1 < j) {
-                    const double u = A[p1 * LD + j];
-#pragma unroll
-                    for (int d = 0; d < D; ++d) y1[d] -= u * xj[d];
-                }
-            }
-            if (has2) {
-                if (lane == j) {
-#pragma unroll
-                    for (int d = 0; d < D; ++d) y2[d] = xj[d];
-                } else if (lane < j) {
-                    const double u = A[lane * LD + j];
-#pragma unroll
-                    for (int d = 0; d < D; ++d) y2[d] -= u * xj[d];
-                }
-            }
-        }
-        // weight of support t = lane: row t sits in lane t - OFF (or in y2)
+        if (sys.solve(k, xs, rhs, pr, rows) && lane == 0) atomicOr(status, 2);
         double W0[D], W1[D];
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-            const double v = __shfl_sync(kFull, y1[d], (lane - OFF) & 31);
-            W0[d] = (lane >= OFF ? v : y2[d]) + (lane == 0 ? cself[d] : 0.0);
+            // the node's own support also carries the [s = 0] term
+            W0[d] = lane < k ? rows[lane * D + d] + (lane == 0 ? tq.ksum[d] * rdel : 0.0) : 0.0;
             W1[d] = 0.0;
         }
-        write_node<D>(out, i, KC, ns, W0, W1);
+        write_node<D>(out, i, k, ns, W0, W1);
         __syncwarp();
     }
+}
+
+// Weights of up to NR queries of a group per solve (the elimination is run
+// again for every NR of them: the caller takes it for groups of at most NR).
+// T: type of the queries and the weights.
+template <int D, int KC, int NR, class T>
+__global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
+    rbf_weights_gj_kernel(const float* __restrict__ src, int64_t nsrc, const uint32_t* __restrict__ support, int k,
+                          const T* __restrict__ qry, int64_t ngroups, int group, double spacing, int shape,
+                          T* __restrict__ weights, int* __restrict__ status) {
+    using S = GjSystem<KC, D, NR>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int w = threadIdx.x >> 5, lane = lane_id();
+    double* rows = reinterpret_cast<double*>(smem) + (size_t)S::doubles * w;
+    double* pr = rows + S::kAsm;
+    double* rhs = pr + S::kRow;
+    double* xs = rhs + S::kRhs;
+    for (int64_t g = (int64_t)blockIdx.x * kGjBlockWarps + w; g < ngroups; g += (int64_t)gridDim.x * kGjBlockWarps) {
+        double o[D], xl[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            o[d] = (double)qry[(g * group) * D + d];
+            xl[d] = 0.0;
+        }
+        if (lane < k) {
+            uint32_t j = support[g * k + lane];
+            if ((int64_t)j >= nsrc) {
+                atomicOr(status, 1);
+                j = 0;
+            }
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                xl[d] = ((double)src[(int64_t)j * D + d] - o[d]) / spacing;
+                xs[lane * D + d] = xl[d];
+            }
+        }
+        __syncwarp();
+        S sys;
+        assemble<D, KC, NR>(sys, xs, k, shape, rows);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            double x[D], r2 = 0;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                x[d] = q < group ? ((double)qry[(g * group + q) * D + d] - o[d]) / spacing : 0.0;
+                const double t = xl[d] - x[d];
+                r2 += t * t;
+            }
+            sys.a[S::E + KC + q] = lane < k ? shape_fn(r2, shape) : 0.0;
+            if (lane == 0) {
+                rhs[q] = 1.0;
+#pragma unroll
+                for (int d = 0; d < D; ++d) rhs[(1 + d) * NR + q] = x[d];
+            }
+        }
+        __syncwarp();
+        if (sys.solve(k, xs, rhs, pr, rows) && lane == 0) atomicOr(status, 2);
+        if (lane < k)
+            for (int q = 0; q < NR && q < group; ++q) weights[(g * group + q) * k + lane] = (T)rows[lane * NR + q];
+        __syncwarp();
+    }
+}
+
+// launches kern over `count` warps' worth of systems with the per-warp shared
+// memory of S
+template <class S, class Kern, class... Args>
+int launch_gj_systems(Kern kern, int64_t count, cudaStream_t st, Args... args) {
+    const size_t smem = sizeof(double) * S::doubles * kGjBlockWarps;
+    NAGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = (int)std::min<int64_t>((count + kGjBlockWarps - 1) / kGjBlockWarps, (int64_t)sm_count() * 32);
+    kern<<<blocks, 32 * kGjBlockWarps, smem, st>>>(args...);
+    NAGA_CUDA_TRY(cudaGetLastError());
+    return NAGA_OK;
+}
+
+// fn(KC as std::integral_constant) for the padded size of a stencil of k <= 32
+template <class Fn>
+int with_padded_size(int k, Fn&& fn) {
+    if (k <= 16) return fn(std::integral_constant<int, 16>{});
+    if (k <= 24) return fn(std::integral_constant<int, 24>{});
+    return fn(std::integral_constant<int, 32>{});
+}
+
+// the register solve serves FP64 systems of up to 32 supports, and groups of
+// up to four queries (beyond that the general kernel's one factorisation
+// serves all of a group)
+bool gj_serves(int k, int group, int precision) { return precision == 0 && k <= 32 && group <= 4; }
+
+template <class T>
+int rbf_weights_gj(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const T* qry,
+                   int64_t ngroups, int group, double spacing, int shape, T* weights, int* status, cudaStream_t st) {
+    return with_padded_size(k, [&](auto kc) -> int {
+        constexpr int KC = decltype(kc)::value;
+        auto go = [&](auto d, auto nr) -> int {
+            constexpr int D = decltype(d)::value, NR = decltype(nr)::value;
+            return launch_gj_systems<GjSystem<KC, D, NR>>(rbf_weights_gj_kernel<D, KC, NR, T>, ngroups, st, src, nsrc,
+                                                          support, k, qry, ngroups, group, spacing, shape, weights,
+                                                          status);
+        };
+        using std::integral_constant;
+        if (dim == 2)
+            return group == 1 ? go(integral_constant<int, 2>{}, integral_constant<int, 1>{})
+                              : go(integral_constant<int, 2>{}, integral_constant<int, 4>{});
+        return group == 1 ? go(integral_constant<int, 3>{}, integral_constant<int, 1>{})
+                          : go(integral_constant<int, 3>{}, integral_constant<int, 4>{});
+    });
+}
+
+__global__ void widen_kernel(const float* __restrict__ in, double* __restrict__ out, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = (double)in[i];
+}
+__global__ void narrow_kernel(const double* __restrict__ in, float* __restrict__ out, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = (float)in[i];
 }
 
 int warps_per_block_for(size_t per_warp) {
@@ -786,10 +812,12 @@ int warps_per_block_for(size_t per_warp) {
 
 }  // namespace
 
-// RBF weights on the device; status bits: 1 bad index, 2 singular, 4 no convergence
-int rbf_weights_device(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const double* qry,
-                       int64_t ngroups, int group, double spacing, int shape, int precision, double* weights,
-                       cudaStream_t st) {
+// RBF weights on the device; status bits: 1 bad index, 2 singular, 4 no convergence.
+// T: type of the queries and the weights; the general kernel takes doubles only.
+template <class T>
+static int rbf_weights_typed(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const T* qry,
+                             int64_t ngroups, int group, double spacing, int shape, int precision, T* weights,
+                             cudaStream_t st) {
     const int n = k + dim + 1;
     if (dim != 2 && dim != 3) return set_error(NAGA_EINVAL, "naga_rbf_weights: dim must be 2 or 3");
     if (k < dim + 1 || n > 64) return set_error(NAGA_EINVAL, "naga_rbf_weights: need dim + 1 <= k <= 60");
@@ -804,16 +832,20 @@ int rbf_weights_device(const float* src, int64_t nsrc, int dim, const uint32_t* 
     int* d_status = nullptr;
     NAGA_CUDA_TRY(scratch_malloc(&d_status, 2 * sizeof(int), st));
     NAGA_CUDA_TRY(cudaMemsetAsync(d_status, 0, 2 * sizeof(int), st));
-    const int blocks = (int)std::min<int64_t>((ngroups + wpb - 1) / wpb, (int64_t)sm_count() * 32);
-    const size_t smem = per_warp * wpb;
-    if (dim == 2) {
-        NAGA_CUDA_TRY(cudaFuncSetAttribute(rbf_weights_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        rbf_weights_kernel<2><<<blocks, 32 * wpb, smem, st>>>(src, nsrc, support, k, qry, ngroups, group, spacing,
-                                                              shape, precision, weights, d_status, wpb);
-    } else {
-        NAGA_CUDA_TRY(cudaFuncSetAttribute(rbf_weights_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        rbf_weights_kernel<3><<<blocks, 32 * wpb, smem, st>>>(src, nsrc, support, k, qry, ngroups, group, spacing,
-                                                              shape, precision, weights, d_status, wpb);
+    if (gj_serves(k, group, precision)) {
+        const int rc = rbf_weights_gj<T>(src, nsrc, dim, support, k, qry, ngroups, group, spacing, shape, weights,
+                                         d_status, st);
+        if (rc) {
+            cudaFreeAsync(d_status, st);
+            return rc;
+        }
+    } else if constexpr (std::is_same<T, double>::value) {
+        const int blocks = (int)std::min<int64_t>((ngroups + wpb - 1) / wpb, (int64_t)sm_count() * 32);
+        const size_t smem = per_warp * wpb;
+        auto kern = dim == 2 ? rbf_weights_kernel<2> : rbf_weights_kernel<3>;
+        NAGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<blocks, 32 * wpb, smem, st>>>(src, nsrc, support, k, qry, ngroups, group, spacing, shape, precision,
+                                             weights, d_status, wpb);
     }
     NAGA_CUDA_TRY(cudaGetLastError());
     int h_st[2] = {0, 0};
@@ -825,6 +857,39 @@ int rbf_weights_device(const float* src, int64_t nsrc, int dim, const uint32_t* 
     if (h_status & 1) return set_error(NAGA_EINVAL, "naga_rbf_weights: support index out of range");
     if (h_status & 2) return set_error(NAGA_ESINGULAR, "naga_rbf_weights: singular moment matrix");
     return NAGA_OK;
+}
+
+int rbf_weights_device(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const double* qry,
+                       int64_t ngroups, int group, double spacing, int shape, int precision, double* weights,
+                       cudaStream_t st) {
+    return rbf_weights_typed<double>(src, nsrc, dim, support, k, qry, ngroups, group, spacing, shape, precision,
+                                     weights, st);
+}
+
+// FP32 queries and weights: read and written by the register solve itself,
+// through FP64 copies for the systems it does not serve
+int rbf_weights_f32_device(const float* src, int64_t nsrc, int dim, const uint32_t* support, int k, const float* qry,
+                           int64_t ngroups, int group, double spacing, int shape, int precision, float* weights,
+                           cudaStream_t st) {
+    if (gj_serves(k, group, precision))
+        return rbf_weights_typed<float>(src, nsrc, dim, support, k, qry, ngroups, group, spacing, shape, precision,
+                                        weights, st);
+    const int64_t nq = ngroups * group;
+    double *q64 = nullptr, *w64 = nullptr;
+    NAGA_CUDA_TRY(scratch_malloc(&q64, sizeof(double) * nq * dim, st));
+    NAGA_CUDA_TRY(scratch_malloc(&w64, sizeof(double) * nq * k, st));
+    const int b1 = (int)std::min<int64_t>((nq * dim + 255) / 256, (int64_t)sm_count() * 8);
+    widen_kernel<<<b1, 256, 0, st>>>(qry, q64, nq * dim);
+    NAGA_CUDA_TRY(cudaGetLastError());
+    int rc = rbf_weights_device(src, nsrc, dim, support, k, q64, ngroups, group, spacing, shape, precision, w64, st);
+    if (rc == NAGA_OK) {
+        const int b2 = (int)std::min<int64_t>((nq * k + 255) / 256, (int64_t)sm_count() * 8);
+        narrow_kernel<<<b2, 256, 0, st>>>(w64, weights, nq * k);
+        if (cudaGetLastError() != cudaSuccess) rc = set_error(NAGA_ECUDA, "naga_rbf_weights_f32: narrow kernel");
+    }
+    cudaFreeAsync(q64, st);
+    cudaFreeAsync(w64, st);
+    return rc;
 }
 
 // kNN + interaction radii + MQ spacing + stencil weights for pts[0, n)
@@ -847,6 +912,10 @@ int divergence_build_device(const float* pts, int64_t n, int dim, int k, int sha
             else
                 quad_table_kernel<3><<<1, 64, 0, st>>>();
             NAGA_CUDA_TRY(cudaGetLastError());
+            void* table = nullptr;
+            NAGA_CUDA_TRY(cudaGetSymbolAddress(&table, g_quad));
+            NAGA_CUDA_TRY(cudaMemcpyToSymbolAsync(c_quad, static_cast<QuadTable*>(table) + (dim - 2), sizeof(QuadTable),
+                                                  sizeof(QuadTable) * (dim - 2), cudaMemcpyDeviceToDevice, st));
             NAGA_CUDA_TRY(cudaStreamSynchronize(st));
             filled[dev][dim - 2] = true;
         }
@@ -876,24 +945,20 @@ int divergence_build_device(const float* pts, int64_t n, int dim, int k, int sha
         batch_mean_kernel<<<(unsigned)nb, 256, 0, st>>>(nn, n, batch, sp);
         NAGA_CUDA_TRY(cudaGetLastError());
     }
-    auto fixed = [&](auto kern, size_t per_warp) -> int {
-        const int wpb = warps_per_block_for(per_warp);
-        const size_t smem = per_warp * wpb;
-        const int blocks = (int)std::min<int64_t>((n + wpb - 1) / wpb, (int64_t)sm_count() * 32);
-        NAGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<blocks, 32 * wpb, smem, st>>>(pts, n, idx, sp, batch, shape, out, d_status, wpb);
-        return NAGA_OK;
-    };
     const size_t per_warp = rbf_smem_per_warp_h(nsys, k, dim, precision);
     const int wpb = warps_per_block_for(per_warp);
     const size_t smem = per_warp * wpb;
     const int blocks = (int)std::min<int64_t>((n + wpb - 1) / wpb, (int64_t)sm_count() * 32);
     int lrc = NAGA_OK;
-    // FP64 builds of the benchmark stencil sizes take the fixed-size kernel
-    if (precision == 0 && dim == 3 && k == 32) {
-        lrc = fixed(divergence_build_fixed_kernel<3, 32>, AugSize<3, 32>::smem_per_warp);
-    } else if (precision == 0 && dim == 2 && k == 16) {
-        lrc = fixed(divergence_build_fixed_kernel<2, 16>, AugSize<2, 16>::smem_per_warp);
+    if (gj_serves(k, 1, precision)) {
+        lrc = with_padded_size(k, [&](auto kc) -> int {
+            constexpr int KC = decltype(kc)::value;
+            if (dim == 2)
+                return launch_gj_systems<GjSystem<KC, 2, 2>>(divergence_build_gj_kernel<2, KC>, n, st, pts, n, idx, k,
+                                                             sp, batch, shape, out, d_status);
+            return launch_gj_systems<GjSystem<KC, 3, 3>>(divergence_build_gj_kernel<3, KC>, n, st, pts, n, idx, k, sp,
+                                                         batch, shape, out, d_status);
+        });
     } else if (dim == 2) {
         NAGA_CUDA_TRY(cudaFuncSetAttribute(divergence_build_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         divergence_build_kernel<2><<<blocks, 32 * wpb, smem, st>>>(pts, n, idx, k, sp, batch, shape, precision, out,
