@@ -1,6 +1,6 @@
 // Batched inverse of small dense matrices, one warp per matrix: FP64
-// Gauss-Jordan in registers for the stencil system sizes (19, 20, 35, 36),
-// FP64 LU in shared memory for any other n <= 64, and FP32 LU with FP64
+// Gauss-Jordan in registers for n <= 48 (the stencil systems among them), FP64
+// LU in shared memory for any other n <= 64, and FP32 factors with FP64
 // residual refinement.
 //
 // Replaces linalg::batched_matrix_inverse (linalg/batched_matrix_inverse.cuh:
@@ -44,9 +44,11 @@ __global__ void inverse_f64_kernel(const double* __restrict__ A, double* __restr
     }
 }
 
-// Register-resident Gauss-Jordan inverse for the stencil system sizes
-// (n = k + D + 1: 19 / 20 for k = 16, 35 / 36 for k = 32). Lane l holds rows
-// l and l + 32 in registers. Each elimination step publishes the scaled pivot
+// Register-resident Gauss-Jordan inverse of systems of up to 48 rows (the
+// stencil systems have n = k + D + 1: 19 / 20 for k = 16, 35 / 36 for k = 32).
+// N is the size the registers are laid out for: the system's own (n = N), or
+// with PAD the next of a few sizes, the rows and columns past n being those of
+// the identity, pivoted last. Lane l holds rows l and l + 32 in registers. Each elimination step publishes the scaled pivot
 // row in shared memory and every lane updates its rows from it, so the n^3
 // multiply-adds are independent register FMAs rather than a chain of
 // shared-memory read-modify-writes.
@@ -65,20 +67,26 @@ __global__ void inverse_f64_kernel(const double* __restrict__ A, double* __restr
 // column enters at register n - 1; after n steps the order is the identity
 // again. The step loop therefore indexes no register by k.
 //
+// Padded sizes against the LU in shared memory they had before: 100,000
+// systems of 24 x 24 2.24 -> 0.63 ms, 20,000 of 45 x 45 4.29 -> 0.87 ms.
 // Measured alternatives, all slower or equal (10^6 systems of 36 x 36 on
 // B200, 18.6 ms for this form): per-row scales instead of rescaling the pivot
 // row (19.6 ms), the next pivot searched while the current step's columns
 // update (19.6-19.9 ms), a vote-and-shuffle fast path for a unique maximum
 // (19.3 ms), the step loop fully unrolled without rotation (25.3 ms at 228
-// registers).
+// registers), per-row scales with the next pivot searched beside the update
+// (23 to 26 ms: 10 warps/SM, or spills at 12), the four rows past the lanes
+// laid across the warp by column instead of as second rows (31 ms: fewer
+// multiply-adds, twice the instructions around them).
 constexpr int kGjWarps = 2;
 
-template <int N>
-__global__ void __launch_bounds__(32 * kGjWarps, (N > 32 ? 5 : 8))
-    inverse_gj_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int64_t batch,
+template <int N, bool PAD>
+__global__ void __launch_bounds__(32 * kGjWarps, (N > 36 ? 4 : N > 32 ? 5 : 8))
+    inverse_gj_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n_, int64_t batch,
                       int* __restrict__ info) {
     constexpr int S = (N + 31) / 32;
     constexpr int NP = (N + 1) & ~1;
+    const int n = PAD ? n_ : N;
     // per warp: the published pivot row (double-buffered by step parity) and
     // the physical row pivoted at each step
     __shared__ __align__(16) double prow[kGjWarps][2][NP];
@@ -86,7 +94,7 @@ __global__ void __launch_bounds__(32 * kGjWarps, (N > 32 ? 5 : 8))
     const int w = threadIdx.x >> 5, lane = lane_id();
     const int64_t nw = (int64_t)gridDim.x * kGjWarps;
     for (int64_t b = (int64_t)blockIdx.x * kGjWarps + w; b < batch; b += nw) {
-        const double* ai = A + b * (int64_t)(N * N);
+        const double* ai = A + b * (int64_t)(n * n);
         double a[S][N];
         int pos[S];
 #pragma unroll
@@ -94,7 +102,7 @@ __global__ void __launch_bounds__(32 * kGjWarps, (N > 32 ? 5 : 8))
             const int r = lane + 32 * s;
             pos[s] = r < N ? r : N;  // N marks a padding row
 #pragma unroll
-            for (int c = 0; c < N; ++c) a[s][c] = r < N ? ai[r + N * c] : 0.0;
+            for (int c = 0; c < N; ++c) a[s][c] = r < n && c < n ? ai[r + n * c] : (PAD && r == c ? 1.0 : 0.0);
         }
         int inf = 0;
 #pragma unroll 1
@@ -161,114 +169,315 @@ __global__ void __launch_bounds__(32 * kGjWarps, (N > 32 ? 5 : 8))
             }
         }
         __syncwarp();
-        double* o = Ainv + b * (int64_t)(N * N);
+        double* o = Ainv + b * (int64_t)(n * n);
 #pragma unroll
         for (int s = 0; s < S; ++s)
-            if (lane + 32 * s < N)
+            if (lane + 32 * s < n)
 #pragma unroll
-                for (int j = 0; j < N; ++j) o[pos[s] + N * rowk[w][j]] = a[s][j];
+                for (int j = 0; j < N; ++j)
+                    if (j < n) o[pos[s] + n * rowk[w][j]] = a[s][j];
         if (info && lane == 0) info[b] = inf;
         __syncwarp();
     }
 }
 
-// FP32 LU, FP64 residual refinement of every column of the inverse.
-__global__ void inverse_f32r_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t batch,
-                                    int max_iter, double tol, int* __restrict__ info, int warps_per_block) {
+// FP32 inverse of one system by Gauss-Jordan in registers, rows lane and
+// lane + 32 of the warp; the scheme of inverse_gj_kernel with the pivot row
+// published as it is and scaled at the end. Af: the FP64 system, column-major with
+// stride NP, identity past n; out: its inverse, column-major, stride NP.
+// prow: NP floats twice; rowk: NP ints. Returns getrf's info.
+template <int NP>
+__device__ int warp_inverse_f32(const double* Af, int n, float* out, float* prow, int* rowk) {
+    constexpr int S = (NP + 31) / 32;
+    const int lane = lane_id();
+    float a[S][NP], scale[S];
+    int pos[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int r = lane + 32 * s;
+        pos[s] = r < NP ? r : NP;
+        scale[s] = 1.f;
+#pragma unroll
+        for (int c = 0; c < NP; ++c) a[s][c] = r < NP ? (float)Af[r + NP * c] : 0.f;
+    }
+    int inf = 0;
+#pragma unroll 1
+    for (int k = 0; k < NP; ++k) {
+        unsigned h = 0u;
+        int bp = NP;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const unsigned v = __float_as_uint(a[s][0]) & 0x7fffffffu;
+            if (pos[s] >= k && pos[s] < NP && (v > h || (v == h && pos[s] < bp))) {
+                h = v;
+                bp = pos[s];
+            }
+        }
+        const unsigned m = __reduce_max_sync(kFull, h);
+        const int bpos = __reduce_min_sync(kFull, h == m ? bp : NP);
+        const bool zero = m == 0u;
+        if (zero && !inf) inf = k + 1;
+        float* const pr = prow + (k & 1) * NP;
+        bool piv[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            piv[s] = pos[s] == bpos;
+            pos[s] = pos[s] == k ? bpos : (piv[s] ? k : pos[s]);
+            if (piv[s]) {
+                rowk[k] = lane + 32 * s;
+#pragma unroll
+                for (int c = 0; c < NP; c += 4)
+                    *reinterpret_cast<float4*>(pr + c) = make_float4(a[s][c], a[s][c + 1], a[s][c + 2], a[s][c + 3]);
+            }
+        }
+        __syncwarp();
+        const float inv = zero ? 0.f : 1.f / pr[0];
+        float f[S], last[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            f[s] = piv[s] ? 0.f : -(a[s][0] * inv);
+            last[s] = piv[s] ? 1.f : f[s];
+            if (piv[s]) scale[s] = inv;
+        }
+#pragma unroll
+        for (int c = 0; c < NP; c += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(pr + c);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                if (c > 0) a[s][c > 0 ? c - 1 : 0] = fmaf(f[s], q.x, a[s][c]);
+                a[s][c] = fmaf(f[s], q.y, a[s][c + 1]);
+                a[s][c + 1] = fmaf(f[s], q.z, a[s][c + 2]);
+                a[s][c + 2] = fmaf(f[s], q.w, a[s][c + 3]);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) a[s][NP - 1] = last[s];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+        if (lane + 32 * s < NP)
+#pragma unroll
+            for (int c = 0; c < NP; ++c) out[pos[s] + NP * rowk[c]] = a[s][c] * scale[s];
+    __syncwarp();
+    return inf > n ? 0 : inf;
+}
+
+// FP32 inverse, FP64 residual refinement of every column of the inverse:
+// X += B (I - A X) with B the FP32 inverse, one column a lane, 32 columns at
+// a time. The column's residual and correction accumulate in registers; A, B
+// and the column's own entries come from shared memory, A and B as broadcasts
+// shared by the warp's columns. A column is done when its correction falls
+// below the tolerance or no longer shrinks by half.
+// 20,000 systems of 36 x 36: 9.70 -> 1.30 ms, of 20 x 20 1.07 -> 0.27 ms, 5,000
+// of 45 x 45 6.27 -> 0.79 ms (before: triangular solves and residuals read and
+// written in shared memory, one dependent chain a lane). Bound by the latency
+// of the shared-memory operands: 7 warps/SM (31 KB a system), a third of the
+// issue slots.
+// A column's refinement: last correction, the one before, and whether it is
+// done -- below the tolerance, or no longer contracting
+struct RefineState {
+    double dlast = INFINITY, dprev = INFINITY, xlast = 0;
+    bool done;
+    __device__ explicit RefineState(bool idle) : done(idle) {}
+    __device__ void update(float dm, double xm, double tol) {
+        dprev = dlast;
+        dlast = (double)dm;
+        xlast = xm;
+        done = dlast <= tol * xm || dlast > 0.5 * dprev;
+    }
+    // last correction within the tolerance, or within 1e-10 of the column
+    // when refinement stagnated at the FP64 residual floor
+    __device__ bool converged(double tol) const { return dlast <= tol * xlast || dlast <= 1e-10 * xlast; }
+};
+template <int NP>
+struct RefineSize {
+    static_assert(NP % 4 == 0, "16-B columns");
+    // A, X (FP64), B, R (FP32), the published rows and their order
+    static constexpr size_t per_warp = (size_t)NP * NP * (8 + 8 + 4 + 4) + NP * (8 + 4) + 32;
+    static constexpr size_t stride = (per_warp + 127) / 128 * 128;
+};
+template <int NP>
+__global__ void __launch_bounds__(NP > 36 ? 128 : 224)
+    inverse_f32r_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t batch, int max_iter,
+                        double tol, int* __restrict__ info, int warps_per_block) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = lane_id();
-    const size_t per_warp = (size_t)24 * n * n + 16 * ((n + 3) / 4);
-    double* Ad = reinterpret_cast<double*>(smem + per_warp * w);
-    double* X = Ad + n * n;
-    float* LUf = reinterpret_cast<float*>(X + n * n);
-    float* R = LUf + n * n;
-    int* piv = reinterpret_cast<int*>(R + n * n);
+    double* Ad = reinterpret_cast<double*>(smem + RefineSize<NP>::stride * w);
+    double* X = Ad + NP * NP;  // X[j NP + c]: row j of column c
+    float* B = reinterpret_cast<float*>(X + NP * NP);
+    float* R = B + NP * NP;    // as X
+    float* prow = R + NP * NP;
+    int* rowk = reinterpret_cast<int*>(prow + 2 * NP);
     const int64_t nw = (int64_t)gridDim.x * warps_per_block;
     for (int64_t b = (int64_t)blockIdx.x * warps_per_block + w; b < batch; b += nw) {
         const double* a = A + b * (int64_t)n * n;
-        for (int e = lane; e < n * n; e += 32) {
-            double v = a[e];
-            Ad[e] = v;
-            LUf[e] = (float)v;
+        for (int e = lane; e < NP * NP; e += 32) {
+            const int r = e % NP, c = e / NP;
+            Ad[e] = r < n && c < n ? a[r + (int64_t)n * c] : (r == c ? 1.0 : 0.0);
         }
         __syncwarp();
-        int inf = warp_lu(LUf, n, piv);
-        warp_lu_inverse(LUf, n, piv, R);
-        for (int e = lane; e < n * n; e += 32) X[e] = (double)R[e];
-        __syncwarp();
-        // per column: last correction, the one before, and whether it is done
-        double dlast[2] = {INFINITY, INFINITY}, dprev[2] = {INFINITY, INFINITY}, xlast[2] = {0, 0};
-        bool cdone[2] = {lane >= n, lane + 32 >= n};
-        bool done = false;
-        for (int it = 0; it < max_iter && !done && inf == 0; ++it) {
-            // residual R = I - A X, column c by lane c
-            for (int c = lane; c < n; c += 32)
-                for (int i = 0; i < n; ++i) {
-                    double r = (i == c) ? 1.0 : 0.0;
-                    for (int j = 0; j < n; ++j) r -= Ad[i + n * j] * X[j * n + c];
-                    R[i * n + c] = (float)r;
-                }
-            __syncwarp();
-            // correction D = LU^-1 R (in place), X += D
-            for (int c = lane, t = 0; c < n; c += 32, ++t) {
-                if (cdone[t]) continue;
+        const int inf = warp_inverse_f32<NP>(Ad, n, B, prow, rowk);
+        bool conv = true;
+        // columns 0 .. 31, one a lane
+        {
+            const int c = lane;
+            const bool has = c < n;
+            const int cc = has ? c : 0;  // idle lanes read column 0
+            if (has)
+                for (int j = 0; j < NP; ++j) X[j * NP + c] = (double)B[j + NP * c];
+            RefineState st(!has);
+            for (int it = 0; it < max_iter && inf == 0 && !__all_sync(kFull, st.done); ++it) {
+                // residual R = I - A X
+                double r[NP];
+#pragma unroll
+                for (int i = 0; i < NP; ++i) r[i] = i == c ? 1.0 : 0.0;
+#pragma unroll 2
                 for (int j = 0; j < n; ++j) {
-                    const int p = piv[j];
-                    if (p != j) {
-                        float tmp = R[j * n + c];
-                        R[j * n + c] = R[p * n + c];
-                        R[p * n + c] = tmp;
+                    const double xj = -X[j * NP + cc];
+                    const double2* col = reinterpret_cast<const double2*>(Ad + NP * j);
+#pragma unroll
+                    for (int i = 0; i < NP; i += 2) {
+                        const double2 v = col[i / 2];
+                        r[i] = fma(v.x, xj, r[i]);
+                        r[i + 1] = fma(v.y, xj, r[i + 1]);
                     }
                 }
+                if (has) {
+#pragma unroll
+                    for (int i = 0; i < NP; ++i) R[i * NP + c] = (float)r[i];
+                }
+                // correction D = B R, X += D
+                float d[NP];
+#pragma unroll
+                for (int i = 0; i < NP; ++i) d[i] = 0.f;
+#pragma unroll 2
                 for (int j = 0; j < n; ++j) {
-                    const float xj = R[j * n + c];
-                    for (int i = j + 1; i < n; ++i) R[i * n + c] -= LUf[i + n * j] * xj;
+                    const float rj = R[j * NP + cc];
+                    const float4* col = reinterpret_cast<const float4*>(B + NP * j);
+#pragma unroll
+                    for (int i = 0; i < NP; i += 4) {
+                        const float4 v = col[i / 4];
+                        d[i] = fmaf(v.x, rj, d[i]);
+                        d[i + 1] = fmaf(v.y, rj, d[i + 1]);
+                        d[i + 2] = fmaf(v.z, rj, d[i + 2]);
+                        d[i + 3] = fmaf(v.w, rj, d[i + 3]);
+                    }
                 }
-                for (int j = n - 1; j >= 0; --j) {
-                    const float xj = R[j * n + c] / LUf[j + n * j];
-                    R[j * n + c] = xj;
-                    for (int i = 0; i < j; ++i) R[i * n + c] -= LUf[i + n * j] * xj;
+                if (!st.done) {
+                    float dm = 0.f;
+                    double xm = 0;
+#pragma unroll
+                    for (int i = 0; i < NP; ++i) {
+                        const double x = X[i * NP + c] + (double)d[i];
+                        X[i * NP + c] = x;
+                        if (i < n) {
+                            dm = fmaxf(dm, fabsf(d[i]));
+                            xm = fmax(xm, fabs(x));
+                        }
+                    }
+                    st.update(dm, xm, tol);
                 }
-                double dmax = 0, xmax = 0;
-                for (int i = 0; i < n; ++i) {
-                    double x = X[i * n + c] + (double)R[i * n + c];
-                    X[i * n + c] = x;
-                    dmax = fmax(dmax, fabs((double)R[i * n + c]));
-                    xmax = fmax(xmax, fabs(x));
-                }
-                dprev[t] = dlast[t];
-                dlast[t] = dmax;
-                xlast[t] = xmax;
-                // done when below the tolerance or no longer contracting
-                cdone[t] = dmax <= tol * xmax || dmax > 0.5 * dprev[t];
             }
-            done = __all_sync(kFull, cdone[0] && cdone[1]);
-            __syncwarp();
+            if (has) conv = st.converged(tol);
         }
-        // converged: last correction within the tolerance, or within 1e-10
-        // of the column when refinement stagnated at the FP64 residual floor
-        bool conv = true;
-        for (int t = 0; t < 2; ++t)
-            if (lane + 32 * t < n)
-                conv = conv && (dlast[t] <= tol * xlast[t] || dlast[t] <= 1e-10 * xlast[t]);
-        done = __all_sync(kFull, conv);
+        __syncwarp();
+        // columns 32 .. n - 1, C at a time, 32 / C lanes a column: lane l
+        // takes rows (l / C) RL .. of column c0 + l % C, so the few columns
+        // past the lanes do not cost another full pass
+        constexpr int C = 4, RL = (NP + 32 / C - 1) / (32 / C);
+        for (int c0 = 32; c0 < n; c0 += C) {
+            const int c = c0 + lane % C, i0 = lane / C * RL;
+            const bool has = c < n;
+            const int cc = has ? c : c0;
+            if (has)
+                for (int u = 0; u < RL; ++u)
+                    if (i0 + u < NP) X[(i0 + u) * NP + c] = (double)B[i0 + u + NP * c];
+            __syncwarp();
+            RefineState st(!has);
+            for (int it = 0; it < max_iter && inf == 0 && !__all_sync(kFull, st.done); ++it) {
+                double r[RL];
+                float d[RL];
+                int row[RL];
+#pragma unroll
+                for (int u = 0; u < RL; ++u) {
+                    row[u] = i0 + u < NP ? i0 + u : NP - 1;
+                    r[u] = row[u] == c ? 1.0 : 0.0;
+                    d[u] = 0.f;
+                }
+#pragma unroll 4
+                for (int j = 0; j < n; ++j) {
+                    const double xj = -X[j * NP + cc];
+#pragma unroll
+                    for (int u = 0; u < RL; ++u) r[u] = fma(Ad[row[u] + NP * j], xj, r[u]);
+                }
+                __syncwarp();
+                if (has) {
+#pragma unroll
+                    for (int u = 0; u < RL; ++u)
+                        if (i0 + u < NP) R[row[u] * NP + c] = (float)r[u];
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (int j = 0; j < n; ++j) {
+                    const float rj = R[j * NP + cc];
+#pragma unroll
+                    for (int u = 0; u < RL; ++u) d[u] = fmaf(B[row[u] + NP * j], rj, d[u]);
+                }
+                float dm = 0.f;
+                double xm = 0;
+#pragma unroll
+                for (int u = 0; u < RL; ++u)
+                    if (!st.done && i0 + u < n) {
+                        const double x = X[row[u] * NP + c] + (double)d[u];
+                        X[row[u] * NP + c] = x;
+                        dm = fmaxf(dm, fabsf(d[u]));
+                        xm = fmax(xm, fabs(x));
+                    }
+#pragma unroll
+                for (int o = C; o < 32; o <<= 1) {
+                    dm = fmaxf(dm, __shfl_xor_sync(kFull, dm, o));
+                    xm = fmax(xm, __shfl_xor_sync(kFull, xm, o));
+                }
+                if (!st.done) st.update(dm, xm, tol);
+                __syncwarp();
+            }
+            if (has) conv = conv && st.converged(tol);
+        }
+        __syncwarp();
+        const bool ok = __all_sync(kFull, conv);
         double* o = Ainv + b * (int64_t)n * n;
-        for (int e = lane; e < n * n; e += 32) o[e] = X[(e % n) * n + e / n];
-        if (info && lane == 0) info[b] = inf != 0 ? inf : (done ? 0 : -1);
+        for (int e = lane; e < n * n; e += 32) o[e] = X[(e % n) * NP + e / n];
+        if (info && lane == 0) info[b] = inf != 0 ? inf : (ok ? 0 : -1);
         __syncwarp();
     }
 }
 
-template <int N>
-int launch_gj(const double* A, double* Ainv, int64_t batch, int* info, cudaStream_t st) {
+template <int NP>
+int launch_f32r(const double* A, double* Ainv, int n, int64_t batch, int max_iter, double tol, int* info,
+                cudaStream_t st) {
+    const size_t stride = RefineSize<NP>::stride;
+    const int wpb = (int)std::min<size_t>(NP > 36 ? 4 : 7, smem_limit() / stride);
+    if (wpb < 1) return set_error(NAGA_EINVAL, "batched inverse: matrix too large for shared memory");
+    const size_t smem = stride * wpb;
+    NAGA_CUDA_TRY(cudaFuncSetAttribute(inverse_f32r_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = (int)std::min<int64_t>((batch + wpb - 1) / wpb, (int64_t)sm_count() * 32);
+    inverse_f32r_kernel<NP><<<blocks, 32 * wpb, smem, st>>>(A, Ainv, n, batch, max_iter, tol, info, wpb);
+    NAGA_CUDA_TRY(cudaGetLastError());
+    return NAGA_OK;
+}
+
+template <int N, bool PAD>
+int launch_gj(const double* A, double* Ainv, int n, int64_t batch, int* info, cudaStream_t st) {
     static int per_sm = 0;
+    auto kern = inverse_gj_kernel<N, PAD>;
     if (per_sm < 1) {
-        NAGA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, inverse_gj_kernel<N>, 32 * kGjWarps, 0));
+        NAGA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kGjWarps, 0));
         per_sm = std::max(per_sm, 1);
     }
     const int64_t need = (batch + kGjWarps - 1) / kGjWarps;
     const int blocks = (int)std::min<int64_t>(need, (int64_t)sm_count() * per_sm);
-    inverse_gj_kernel<N><<<blocks, 32 * kGjWarps, 0, st>>>(A, Ainv, batch, info);
+    kern<<<blocks, 32 * kGjWarps, 0, st>>>(A, Ainv, n, batch, info);
     NAGA_CUDA_TRY(cudaGetLastError());
     return NAGA_OK;
 }
@@ -281,27 +490,38 @@ int batched_inverse(const double* A, double* Ainv, int n, int64_t batch, int* in
     if (batch < 0) return set_error(NAGA_EINVAL, "batched inverse: negative batch");
     if (batch == 0) return NAGA_OK;
     if (!A || !Ainv) return set_error(NAGA_EINVAL, "batched inverse: null pointer");
-    if (!refined) switch (n) {
-            case 19: return launch_gj<19>(A, Ainv, batch, info, st);
-            case 20: return launch_gj<20>(A, Ainv, batch, info, st);
-            case 35: return launch_gj<35>(A, Ainv, batch, info, st);
-            case 36: return launch_gj<36>(A, Ainv, batch, info, st);
+    // up to 48 rows in registers: the stencil systems at their own size, the
+    // others rounded up to the next of a few; larger ones by LU in shared
+    // memory
+    if (!refined && n <= 48) {
+        switch (n) {
+            case 19: return launch_gj<19, false>(A, Ainv, n, batch, info, st);
+            case 20: return launch_gj<20, false>(A, Ainv, n, batch, info, st);
+            case 35: return launch_gj<35, false>(A, Ainv, n, batch, info, st);
+            case 36: return launch_gj<36, false>(A, Ainv, n, batch, info, st);
             default: break;
         }
-    const size_t per_warp = (refined ? (size_t)24 : (size_t)16) * n * n + 16 * ((n + 3) / 4);
-    const size_t lim = smem_limit();
-    int wpb = (int)std::min<size_t>(8, lim / per_warp);
+        if (n <= 8) return launch_gj<8, true>(A, Ainv, n, batch, info, st);
+        if (n <= 16) return launch_gj<16, true>(A, Ainv, n, batch, info, st);
+        if (n <= 24) return launch_gj<24, true>(A, Ainv, n, batch, info, st);
+        if (n <= 32) return launch_gj<32, true>(A, Ainv, n, batch, info, st);
+        return launch_gj<48, true>(A, Ainv, n, batch, info, st);
+    }
+    if (refined) {
+        if (n <= 20) return launch_f32r<20>(A, Ainv, n, batch, max_iter, tol, info, st);
+        if (n <= 28) return launch_f32r<28>(A, Ainv, n, batch, max_iter, tol, info, st);
+        if (n <= 36) return launch_f32r<36>(A, Ainv, n, batch, max_iter, tol, info, st);
+        if (n <= 48) return launch_f32r<48>(A, Ainv, n, batch, max_iter, tol, info, st);
+        return launch_f32r<64>(A, Ainv, n, batch, max_iter, tol, info, st);
+    }
+    const size_t per_warp = (size_t)16 * n * n + 16 * ((n + 3) / 4);
+    const int wpb = (int)std::min<size_t>(8, smem_limit() / per_warp);
     if (wpb < 1) return set_error(NAGA_EINVAL, "batched inverse: matrix too large for shared memory");
     const size_t smem = per_warp * wpb;
     const int64_t blocks_needed = (batch + wpb - 1) / wpb;
     const int blocks = (int)std::min<int64_t>(blocks_needed, (int64_t)sm_count() * 32);
-    if (!refined) {
-        NAGA_CUDA_TRY(cudaFuncSetAttribute(inverse_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        inverse_f64_kernel<<<blocks, 32 * wpb, smem, st>>>(A, Ainv, n, batch, info, wpb);
-    } else {
-        NAGA_CUDA_TRY(cudaFuncSetAttribute(inverse_f32r_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        inverse_f32r_kernel<<<blocks, 32 * wpb, smem, st>>>(A, Ainv, n, batch, max_iter, tol, info, wpb);
-    }
+    NAGA_CUDA_TRY(cudaFuncSetAttribute(inverse_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    inverse_f64_kernel<<<blocks, 32 * wpb, smem, st>>>(A, Ainv, n, batch, info, wpb);
     NAGA_CUDA_TRY(cudaGetLastError());
     return NAGA_OK;
 }

@@ -170,6 +170,24 @@ def test_inverse_rbf_systems_f64_and_refined(naga, oracle):
     assert er.max() < 1e-10
 
 
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16, 17, 21, 24, 28, 29, 32, 33, 36, 37, 45, 48, 49])
+def test_inverse_every_register_size(naga, oracle, n):
+    """The sizes at and beside those the register kernels are laid out for, a
+    ragged batch of systems (one more than a block's share) in FP64 and in
+    refined FP32, within a small multiple of eps cond(A) of the oracle (the
+    refined inverse stops at the rounding of the n-term FP64 residuals)."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((37, n, n)) + np.eye(n) * 2
+    ref, _ = oracle.batched_inverse(A)
+    out, info = naga.batched_inverse_f64(_t(A))
+    assert (_np(info) == 0).all()
+    _assert_inverse_close(_np(out), ref, A)
+    out, info = naga.batched_inverse_f32r(_t(A), max_iter=30)
+    assert (_np(info) == 0).all()
+    err = np.abs(_np(out) - ref).max(axis=(1, 2)) / np.abs(ref).max(axis=(1, 2))
+    assert (err <= (4 + n) * np.finfo(np.float64).eps * np.linalg.cond(A)).all()
+
+
 def test_inverse_refined_flags_hopeless_systems(naga):
     """Condition ~1e12 is beyond FP32 refinement: flagged (-1), not silent."""
     rng = np.random.default_rng(1)
@@ -179,6 +197,29 @@ def test_inverse_refined_flags_hopeless_systems(naga):
     A = (U @ np.diag(np.logspace(0, -12, n)) @ V.T)[None].repeat(4, 0)
     _, info = naga.batched_inverse_f32r(_t(A.transpose(0, 2, 1).copy()), max_iter=10)
     assert (_np(info) == -1).all()
+
+
+@pytest.mark.parametrize("dim,k,group", [(2, 4, 1), (2, 15, 2), (2, 16, 4), (2, 17, 1), (2, 25, 5), (2, 32, 1),
+                                         (3, 5, 1), (3, 16, 3), (3, 24, 1), (3, 25, 4), (3, 31, 5), (3, 32, 1),
+                                         (3, 33, 1)])
+def test_rbf_weights_every_padded_size(naga, oracle, dim, k, group):
+    """Stencil sizes at and beside the register solve's (16, 24, 32) and past
+    it, groups of queries it serves and one larger, FP64 and FP32 outputs."""
+    rng = np.random.default_rng(100 * dim + k)
+    m = 8 if dim == 3 else 20
+    h = 1.0 / (m - 1)
+    g = np.stack(np.meshgrid(*[np.arange(m) * h] * dim, indexing="ij"), -1).reshape(-1, dim)
+    pts = (g + rng.uniform(-0.25 * h, 0.25 * h, g.shape)).astype(np.float32)
+    centre = rng.random((101, dim)) * 0.8 + 0.1
+    sup, _ = oracle.knn(pts, centre.astype(np.float32), k)
+    qry = (centre[:, None] + rng.uniform(-0.2 * h, 0.2 * h, (101, group, dim))).reshape(-1, dim).astype(np.float32)
+    ref = oracle.rbf_weights(pts, sup, qry.astype(np.float64), group, float(np.float32(h)), 0)
+    w = _np(naga.rbf_weights(_t(pts), _t(sup.astype(np.int32)), _t(qry.astype(np.float64)), group,
+                             float(np.float32(h)), 0))
+    scale = np.abs(ref).max()
+    assert np.abs(w - ref).max() <= 1e-10 * scale
+    w32 = _np(naga.rbf_weights_f32(_t(pts), _t(sup.astype(np.int32)), _t(qry), group, float(np.float32(h)), 0))
+    assert np.abs(w32 - ref).max() <= 1.2e-7 * scale
 
 
 @pytest.mark.parametrize("dim,shape,precision", [(2, 0, 0), (2, 1, 0), (3, 0, 0), (3, 1, 0), (3, 1, 1)])
