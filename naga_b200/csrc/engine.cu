@@ -197,6 +197,43 @@ __global__ void boundary_records_kernel(const uint32_t* __restrict__ idx, const 
     is_src[j] = 1;
 }
 
+// Results of a scene in the layout its reader asked for, so that they go to
+// the host as they are (rearranged on the host, the populations of a 10k-node
+// 3-D scene took 1.7 ms and the macros of a 1M-node scene 11 ms).
+// Populations in lattice order, one thread a value.
+template <class L>
+__global__ void read_state_kernel(const float* __restrict__ G, int64_t n, float* __restrict__ out) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * L::Q; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e / L::Q;
+        out[e] = G[i * L::QP + L::pos((int)(e - i * L::Q))];
+    }
+}
+// density perturbation: the populations' sum in lattice order, FP64
+template <class L>
+__global__ void read_drho_kernel(const float* __restrict__ G, int64_t n, double rho0, float* __restrict__ out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double r = 0;
+#pragma unroll
+        for (int a = 0; a < L::Q; ++a) r += G[i * L::QP + L::pos(a)];
+        out[i] = (float)(r * rho0);
+    }
+}
+// NAGA stores the macros dimensional: rho rho0 and u c / c_s
+// (detail/simulation_engine.cuh:53-82); the bounce-back of the step resets the
+// boundary nodes' [b0, b1) stored velocity to 0 (:874-877)
+template <int D>
+__global__ void read_macros_kernel(const float4* __restrict__ M, int64_t n, int64_t b0, int64_t b1, double rho0,
+                                   double uscale, float* __restrict__ density, float* __restrict__ velocity) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float4 v = M[i];
+        density[i] = (float)((1.0 + (double)v.x) * rho0);
+        const bool wall = i >= b0 && i < b1;
+        const float u[3] = {v.y, v.z, v.w};
+#pragma unroll
+        for (int d = 0; d < D; ++d) velocity[i * D + d] = wall ? 0.f : (float)((double)u[d] * uscale);
+    }
+}
+
 // the largest layer-support count of each PML item's nodes (the count of
 // node i rides in the bits of PV[2 i].w): the item's PML tile only needs
 // that many records per node
@@ -1133,19 +1170,29 @@ extern "C" int naga_scene_load(naga_scene* s, const void* buf, int64_t size) {
 
 extern "C" int naga_scene_read_state(naga_scene* s, float* g, float* drho) {
     if (!s) return set_error(NAGA_EINVAL, "naga_scene_read_state: null scene");
-    NAGA_CUDA_TRY(cudaStreamSynchronize(active_stream(s)));
-    const int Q = s->Q, QP = s->QP;
-    std::vector<float> buf((size_t)s->N * QP);
-    NAGA_CUDA_TRY(cudaMemcpy(buf.data(), s->dev.G, sizeof(float) * buf.size(), cudaMemcpyDeviceToHost));
-    for (int64_t i = 0; i < s->N; ++i) {
-        double r = 0;
-        for (int a = 0; a < Q; ++a) {
-            float v = buf[(size_t)i * QP + slot_of(s->dim, a)];
-            if (g) g[i * Q + a] = v;
-            r += v;
-        }
-        if (drho) drho[i] = (float)(r * s->desc.rho0);
+    cudaStream_t st = active_stream(s);
+    const int64_t n = s->N;
+    // the collision scratch S1, S1P holds the results (no step reads it before
+    // writing it): work and copies are ordered behind the steps queued
+    float *og = s->dev.S1, *od = s->dev.S1P;
+    const unsigned blocks = (unsigned)std::min<int64_t>((n * s->Q + 255) / 256, (int64_t)sm_count() * 16);
+    if (g && n > 0) {
+        if (s->dim == 2)
+            read_state_kernel<D2Q9><<<blocks, 256, 0, st>>>(s->dev.G, n, og);
+        else
+            read_state_kernel<D3Q27><<<blocks, 256, 0, st>>>(s->dev.G, n, og);
+        NAGA_CUDA_TRY(cudaGetLastError());
+        NAGA_CUDA_TRY(cudaMemcpyAsync(g, og, sizeof(float) * n * s->Q, cudaMemcpyDeviceToHost, st));
     }
+    if (drho && n > 0) {
+        if (s->dim == 2)
+            read_drho_kernel<D2Q9><<<blocks, 256, 0, st>>>(s->dev.G, n, s->desc.rho0, od);
+        else
+            read_drho_kernel<D3Q27><<<blocks, 256, 0, st>>>(s->dev.G, n, s->desc.rho0, od);
+        NAGA_CUDA_TRY(cudaGetLastError());
+        NAGA_CUDA_TRY(cudaMemcpyAsync(drho, od, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
+    }
+    NAGA_CUDA_TRY(cudaStreamSynchronize(st));
     return NAGA_OK;
 }
 
@@ -1171,25 +1218,26 @@ extern "C" int naga_lattice(int dim, int* q, float* weights, int* velocities) {
 
 extern "C" int naga_scene_read_macros(naga_scene* s, float* density, float* velocity) {
     if (!s) return set_error(NAGA_EINVAL, "naga_scene_read_macros: null scene");
-    NAGA_CUDA_TRY(cudaStreamSynchronize(active_stream(s)));
-    std::vector<float4> m((size_t)s->N);
-    NAGA_CUDA_TRY(cudaMemcpy(m.data(), s->dev.M, sizeof(float4) * m.size(), cudaMemcpyDeviceToHost));
-    // NAGA stores the macros dimensional: rho rho0 and u c / c_s
-    // (detail/simulation_engine.cuh:53-82)
-    const double rho0 = s->desc.rho0;
-    const double uscale = s->desc.speed_of_sound / (double)lattice_cs_f();
+    cudaStream_t st = active_stream(s);
+    const int64_t n = s->N;
     const int D = s->dim;
-    for (int64_t i = 0; i < s->N; ++i) {
-        const float4 v = m[(size_t)i];
-        if (density) density[i] = (float)((1.0 + (double)v.x) * rho0);
-        if (velocity) {
-            // the bounce-back of the step resets the boundary nodes' stored
-            // velocity to 0 (detail/simulation_engine.cuh:874-877)
-            const bool wall = i >= s->nbl && i < s->nbl + s->nbd;
-            const float u[3] = {v.y, v.z, v.w};
-            for (int d = 0; d < D; ++d) velocity[i * D + d] = wall ? 0.f : (float)((double)u[d] * uscale);
-        }
+    const double uscale = s->desc.speed_of_sound / (double)lattice_cs_f();
+    // density and velocity side by side in the collision scratch S1, which no
+    // step reads before writing it
+    float *od = s->dev.S1, *ov = s->dev.S1 + n;
+    if (n > 0) {
+        const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 16);
+        if (D == 2)
+            read_macros_kernel<2><<<blocks, 256, 0, st>>>(s->dev.M, n, s->nbl, s->nbl + s->nbd, s->desc.rho0, uscale, od,
+                                                          ov);
+        else
+            read_macros_kernel<3><<<blocks, 256, 0, st>>>(s->dev.M, n, s->nbl, s->nbl + s->nbd, s->desc.rho0, uscale, od,
+                                                          ov);
+        NAGA_CUDA_TRY(cudaGetLastError());
+        if (density) NAGA_CUDA_TRY(cudaMemcpyAsync(density, od, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
+        if (velocity) NAGA_CUDA_TRY(cudaMemcpyAsync(velocity, ov, sizeof(float) * n * D, cudaMemcpyDeviceToHost, st));
     }
+    NAGA_CUDA_TRY(cudaStreamSynchronize(st));
     return NAGA_OK;
 }
 
