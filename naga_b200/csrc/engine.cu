@@ -143,8 +143,11 @@ struct naga_batch {
     WorkItem *d_all = nullptr, *d_all_mt = nullptr, *d_fluid = nullptr, *d_edge = nullptr, *d_pml = nullptr;
     int n_all = 0, n_all_mt = 0, n_fluid = 0, n_edge = 0, n_pml = 0;
     int k = 0, kb = 0;  // common stencil sizes of the members (0 if they differ)
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    // one step, and kGraphSteps of them (long runs)
+    cudaGraph_t graph = nullptr, run_graph = nullptr;
+    cudaGraphExec_t exec = nullptr, run_exec = nullptr;
+    int64_t replays = 0;     // steps replayed since the graph was captured
+    bool run_tried = false;  // run_exec captured, or not to be had
     // grow-only device tables (a membership change rewrites them in place on
     // the batch stream; they are reallocated only when they must grow)
     WorkItem* d_items = nullptr;  // the five item lists back to back
@@ -157,8 +160,12 @@ struct naga_batch {
     void free_graph() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        exec = nullptr;
-        graph = nullptr;
+        if (run_exec) cudaGraphExecDestroy(run_exec);
+        if (run_graph) cudaGraphDestroy(run_graph);
+        exec = run_exec = nullptr;
+        graph = run_graph = nullptr;
+        replays = 0;
+        run_tried = false;
     }
     void free_tables() {
         free_graph();
@@ -725,6 +732,24 @@ StepLaunch launch_of(naga_batch* b) {
     return P;
 }
 
+// `steps` steps as a graph
+int capture_steps(naga_batch* b, int steps, cudaGraph_t* graph, cudaGraphExec_t* exec) {
+    const StepLaunch P = launch_of(b);
+    NAGA_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = NAGA_OK;
+    for (int n = 0; n < steps && rc == NAGA_OK; ++n) rc = enqueue_step(b->dim, b->k, b->kb, P, b->stream);
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(b->stream, &g);
+    if (rc) {
+        if (g) cudaGraphDestroy(g);
+        return rc;
+    }
+    if (e != cudaSuccess) return set_error(NAGA_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    *graph = g;
+    NAGA_CUDA_TRY(cudaGraphInstantiate(exec, g, 0));
+    return NAGA_OK;
+}
+
 // rebuilds the batch's item lists after a membership change, tunes the
 // launch shape of a new batch shape and captures the step graph, so that
 // the next batch_step only launches
@@ -732,35 +757,49 @@ int batch_prepare(naga_batch* b) {
     if (b->members.empty()) return NAGA_OK;
     int rc;
     if (b->dirty && (rc = batch_rebuild(b))) return rc;
-    StepLaunch P = launch_of(b);
-    if (!b->exec && (rc = tune_step_shapes(b->dim, b->k, b->kb, P, b->stream))) return rc;
-    if (!b->exec && !prof_on()) {
-        NAGA_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        rc = enqueue_step(b->dim, b->k, b->kb, P, b->stream);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-        if (rc) {
-            if (g) cudaGraphDestroy(g);
-            return rc;
-        }
-        if (e != cudaSuccess) return set_error(NAGA_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-        b->graph = g;
-        NAGA_CUDA_TRY(cudaGraphInstantiate(&b->exec, g, 0));
-    }
+    if (!b->exec && (rc = tune_step_shapes(b->dim, b->k, b->kb, launch_of(b), b->stream))) return rc;
+    if (!b->exec && !prof_on()) return capture_steps(b, 1, &b->graph, &b->exec);
     return NAGA_OK;
 }
+
+// Long runs replay a graph of several steps. Between two graphs the GPU drains
+// and the next step's first kernel starts from scratch; within one it is
+// launched like the step's other kernels, its prologue beside the kernel
+// before it. A step of 2k nodes in 2-D 32.9 -> 31.6 us, 20k nodes 39.1 -> 36.5,
+// 10k in 3-D about 2 us less, 250k 480 -> 478 (4 steps a graph save two thirds
+// to all of it, 20 no more than 10).
+constexpr int kGraphSteps = 10;
+// Steps replayed one by one before that graph is captured: the capture takes
+// 0.4 to 0.7 ms, what it saves on about 250 steps, which a batch stepped a few
+// times between membership changes would not get back.
+constexpr int64_t kRunAfter = 128;
 
 int batch_step(naga_batch* b, int nsteps) {
     if (nsteps < 0) return set_error(NAGA_EINVAL, "step: negative step count");
     if (b->members.empty() || nsteps == 0) return NAGA_OK;
     int rc;
     if ((rc = batch_prepare(b))) return rc;
-    StepLaunch P = launch_of(b);
     if (prof_on()) {
+        const StepLaunch P = launch_of(b);
         for (int n = 0; n < nsteps; ++n)
             if ((rc = enqueue_step(b->dim, b->k, b->kb, P, b->stream))) return rc;
     } else {
-        for (int n = 0; n < nsteps; ++n) NAGA_CUDA_TRY(cudaGraphLaunch(b->exec, b->stream));
+        int left = nsteps;
+        if (!b->run_tried && b->replays >= kRunAfter && left >= kGraphSteps) {
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(b->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+                b->run_tried = true;
+                // without it (no memory for it, say) the step graph goes on
+                if (capture_steps(b, kGraphSteps, &b->run_graph, &b->run_exec)) {
+                    cudaGetLastError();
+                    b->run_exec = nullptr;
+                }
+            }
+        }
+        if (b->run_exec)
+            for (; left >= kGraphSteps; left -= kGraphSteps) NAGA_CUDA_TRY(cudaGraphLaunch(b->run_exec, b->stream));
+        for (; left > 0; --left) NAGA_CUDA_TRY(cudaGraphLaunch(b->exec, b->stream));
+        b->replays += nsteps;
     }
     for (auto* s : b->members) s->steps += nsteps;
     return NAGA_OK;

@@ -309,6 +309,35 @@ def test_velocity_error_of_3d_scenes(naga, oracle, n_side, steps, bound):
     assert np.mean(errs) < bound, errs
 
 
+@pytest.mark.parametrize("dim,n_side,layers", [(2, 25, 3), (3, 10, 2)])
+def test_long_runs_equal_single_steps(naga, dim, n_side, layers):
+    """After some steps a batch replays long runs as graphs of several steps.
+    Runs of every length around a graph's give the same state and probes, bit
+    for bit, as single steps, and so they do after a membership change."""
+    g = naga.generate_grid(dim, n_side, layers, 5)
+    drho = naga.gaussian_pulse(g["points"], [0.5] * dim, 1e-3, 0.08)
+    scenes = [naga.Scene(g, k=16 if dim == 2 else 32, shape=1 if dim == 2 else 0, probe_capacity=1024,
+                         probes=(PROBES2 if dim == 2 else PROBES3)) for _ in range(3)]
+    for s in scenes:
+        s.set_density(drho)
+    runs, single, other = scenes
+    b = naga.Batch(dim)
+    b.add(runs)
+    total = 0
+    for n in (130, 9, 10, 11, 37, 1):
+        b.step(n)
+        total += n
+    b.add(other)
+    for n in (128, 30):
+        b.step(n)
+        total += n
+    for _ in range(total):
+        single.step(1)
+    assert np.array_equal(runs.state()[0], single.state()[0])
+    assert np.array_equal(runs.probes(0, total), single.probes(0, total))
+    b.close()
+
+
 def test_async_probe_reads_match_synchronous(naga, oracle):
     """Probe samples queued every step behind the step (page-locked host
     buffer, one sync at the end) equal the synchronous read, including a
