@@ -446,13 +446,26 @@ __device__ __forceinline__ void collide(const float* g, float drho, const float*
 // Programmatic dependent launch between the step's kernels: a kernel lets
 // the next one be scheduled once all its blocks have finished their work
 // (earlier, the waiting blocks of later kernels took SM slots from the
-// running one), and the next kernel's blocks run their prologue -- shared-memory set-up and the first
+// running one; a grid of few blocks, see kFewBlocks, does so from its start),
+// and the next kernel's blocks run their prologue -- shared-memory set-up and the first
 // bulk copy of table records, which no kernel of the step writes -- before
 // waiting for the previous kernel's completion and memory (griddepcontrol.
 // wait) ahead of their first read of step data. Without a programmatic
 // dependency (a plain launch) the wait returns at once.
 __device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel whose blocks leave at least half of the SMs free lets the next one
+// be scheduled at once: that one's launch latency then passes beside the whole
+// kernel, and its waiting blocks find slots of their own (all blocks of this
+// grid run by then). Bound by latency, a step of 2k nodes in 2-D takes 31.6 ->
+// 28.1 us, 20k nodes 36.4 -> 33.3, 250k in 3-D 477 -> 475 (its tail and
+// boundary kernels). Up to 148 blocks gave the same, up to 296 a step of 10k
+// nodes in 3-D 50 -> 54 us, and two such scenes on streams of their own lost
+// 3 % at 148, 18 % at 296: the waiting blocks of one keep the other's out.
+constexpr unsigned kFewBlocks = 74;
+__device__ __forceinline__ void pdl_allow_next_if_few() {
+    if (gridDim.x * gridDim.y <= kFewBlocks) pdl_allow_next();
+}
 
 __device__ __forceinline__ void load_scene(SceneDev& dst, const SceneDev* src) {
     if (threadIdx.x < 32) {
@@ -473,6 +486,7 @@ __device__ __forceinline__ void load_scene(SceneDev& dst, const SceneDev* src) {
 template <int QP>
 __global__ void __launch_bounds__(256) k_scene_tail(const SceneDev* __restrict__ scenes) {
     __shared__ double red[256];
+    pdl_allow_next_if_few();
     pdl_wait_prev();
     const SceneDev& S = scenes[blockIdx.x];
     const int t = blockIdx.y;
@@ -667,6 +681,7 @@ __global__ void __launch_bounds__(kBlock, (L::D == 3 ? 4 : 8)) k_macro_pml(const
     WorkItem it = (int)blockIdx.x < nitems ? items[blockIdx.x] : WorkItem{0u, 0u, 0u, 0u};
     if ((int)blockIdx.x < nitems) load_scene(S, scenes + it.scene);
     __syncthreads();
+    pdl_allow_next_if_few();
     pdl_wait_prev();
     for (int w_ = blockIdx.x; w_ < nitems;) {
         const unsigned long long step = *S.step;
@@ -898,6 +913,7 @@ constexpr int tile_cap() {
         if (threadIdx.x == 0) pipe_issue_(pipe_it_, 0);                                                \
         load_scene(pipe_S_[0], scenes + pipe_it_.scene);                                               \
     }                                                                                                  \
+    pdl_allow_next_if_few();                                                                           \
     pdl_wait_prev();                                                                                   \
     if ((int)blockIdx.x < nitems) pipe_wait_(0);                                                       \
     int pipe_t_ = 0;                                                                                   \
@@ -1416,6 +1432,7 @@ __global__ void __launch_bounds__(256, 2) k_rk_halo(const WorkItem* __restrict__
         scene_even = w0.scene;
         load_scene(S2[0], scenes + w0.scene);
     }
+    pdl_allow_next_if_few();
     pdl_wait_prev();
     if (T > 0) {
         wait_blob(0);
