@@ -2073,6 +2073,9 @@ int enqueue_step_k(const StepLaunch& P, cudaStream_t st) {
 // and by 1% otherwise. NAGA_GATHER_BPS=<n> and NAGA_GATHER_TPN=<t> fix the
 // choice instead (bps 0: default carveout; tpn 0 or unlisted: the default;
 // tpn "halo": the halo stages).
+// Trials are launched as the step launches its kernels (PDL): launched plainly,
+// kernels of a few us took 6.6, 8.6 or 10.7 us whatever their work, and a
+// scene of 10k nodes in 3-D fell on a shape of 50 us a step or one of 59.
 template <class L, int K, int KB>
 int tune_k(const StepLaunch& P, cudaStream_t st) {
     if (P.n_fluid <= 0) return NAGA_OK;
@@ -2104,6 +2107,7 @@ int tune_k(const StepLaunch& P, cudaStream_t st) {
         return NAGA_OK;
     }
     const int sms = sm_count();
+    constexpr int kShortReps = 24;  // launches of a trial of a few us each
     cudaEvent_t e0, e1;
     NAGA_CUDA_TRY(cudaEventCreate(&e0));
     NAGA_CUDA_TRY(cudaEventCreate(&e1));
@@ -2125,18 +2129,22 @@ int tune_k(const StepLaunch& P, cudaStream_t st) {
             int maxr = 0;
             NAGA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxr, kern, blk, sm));
             maxr = std::max(maxr, halo ? rk_bps(tpn, 0) : 1);
+            const int resident = maxr;
+            // all items resident at once: no carveout to trade blocks for
+            if (!halo && P.n_fluid <= maxr * sms) maxr = 1;
             std::snprintf(line, sizeof line, " | tpn %s", shape_name<L>(tpn).c_str());
             log += line;
             for (int bps = halo ? rk_bps(tpn, 0) : 0; bps <= maxr; bps = bps == 0 ? 2 : bps + 1) {
                 if ((r = set_blocks_per_sm(kern, sm, bps))) return r;
-                const int g = std::min(P.n_fluid, (bps > 0 ? bps : maxr) * sms);
+                const int g = std::min(P.n_fluid, (bps > 0 ? bps : resident) * sms);
                 // one untimed and one timed launch; launches shorter than
                 // ~0.4 ms are timed again over enough repetitions to span ~2 ms
                 auto timed = [&](int reps, float* ms) -> bool {
                     cudaEventRecord(e0, st);
-                    for (int q = 0; q < reps; ++q) kern<<<g, blk, sm, st>>>(P.fluid, P.n_fluid, P.scenes);
+                    for (int q = 0; q < reps && terr == cudaSuccess; ++q)
+                        terr = launch_step_kernel(kern, g, blk, sm, st, P.fluid, P.n_fluid, P.scenes);
                     cudaEventRecord(e1, st);
-                    terr = cudaEventSynchronize(e1);
+                    if (terr == cudaSuccess) terr = cudaEventSynchronize(e1);
                     if (terr == cudaSuccess) terr = cudaGetLastError();
                     if (terr != cudaSuccess) return false;
                     cudaEventElapsedTime(ms, e0, e1);
@@ -2146,10 +2154,10 @@ int tune_k(const StepLaunch& P, cudaStream_t st) {
                 kern<<<g, blk, sm, st>>>(P.fluid, P.n_fluid, P.scenes);
                 float ms = 0.f, ms2 = 0.f;
                 bool ok = timed(1, &ms);
-                if (ok && ms < 0.4f) ok = timed(std::min(8, std::max(2, (int)(2.f / std::max(ms, 1e-3f)))), &ms);
+                if (ok && ms < 0.4f) ok = timed(std::min(kShortReps, std::max(2, (int)(2.f / std::max(ms, 1e-3f)))), &ms);
                 // twice, the faster kept: other streams' work (a server's
                 // scene set-up) can slow a single trial
-                const int reps2 = ms < 0.4f ? std::min(8, std::max(2, (int)(2.f / std::max(ms, 1e-3f)))) : 1;
+                const int reps2 = ms < 0.4f ? std::min(kShortReps, std::max(2, (int)(2.f / std::max(ms, 1e-3f)))) : 1;
                 if (ok && timed(reps2, &ms2)) ms = std::min(ms, ms2);
                 if (!ok)
                     return set_error(NAGA_ECUDA,
@@ -2197,16 +2205,19 @@ int tune_k(const StepLaunch& P, cudaStream_t st) {
             return;
         }
         maxr = std::max(maxr, 1);
+        const int resident = maxr;
+        if (n <= maxr * sms) maxr = 1;
         log += " | ";
         log += name;
         for (int bps = 0; bps <= maxr; bps = bps == 0 ? 2 : bps + 1) {
             if ((rc = set_blocks_per_sm(kern, smem, bps))) return;
-            const int g = std::min(n, (bps > 0 ? bps : maxr) * sms);
+            const int g = std::min(n, (bps > 0 ? bps : resident) * sms);
             auto timed = [&](int reps, float* ms) -> bool {
                 cudaEventRecord(e0, st);
-                for (int q = 0; q < reps; ++q) kern<<<g, block, smem, st>>>(list, n, P.scenes);
+                for (int q = 0; q < reps && terr == cudaSuccess; ++q)
+                    terr = launch_step_kernel(kern, g, block, smem, st, list, n, P.scenes);
                 cudaEventRecord(e1, st);
-                terr = cudaEventSynchronize(e1);
+                if (terr == cudaSuccess) terr = cudaEventSynchronize(e1);
                 if (terr == cudaSuccess) terr = cudaGetLastError();
                 if (terr != cudaSuccess) return false;
                 cudaEventElapsedTime(ms, e0, e1);
@@ -2216,7 +2227,7 @@ int tune_k(const StepLaunch& P, cudaStream_t st) {
             kern<<<g, block, smem, st>>>(list, n, P.scenes);
             float ms = 0.f, ms2 = 0.f;
             bool ok = timed(1, &ms);
-            const int reps2 = ms < 0.4f ? std::min(8, std::max(2, (int)(2.f / std::max(ms, 1e-3f)))) : 1;
+            const int reps2 = ms < 0.4f ? std::min(kShortReps, std::max(2, (int)(2.f / std::max(ms, 1e-3f)))) : 1;
             if (ok && timed(reps2, &ms2)) ms = std::min(ms, ms2);
             if (!ok) {
                 rc = set_error(NAGA_ECUDA,
