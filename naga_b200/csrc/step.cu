@@ -123,9 +123,6 @@ __device__ __forceinline__ void pair_dirs(int c, float* d0, float* d1) {
     }
 }
 
-// lattice speed of sound as the reference spells it (lattices.cuh:46-49)
-__device__ __forceinline__ float cs_f() { return 0.57735026918962576450914878050196f; }
-
 // full row (QP floats) of node i, slot order
 template <class L>
 __device__ __forceinline__ void store_row(float* base, int64_t i, const float* v) {
@@ -134,7 +131,7 @@ __device__ __forceinline__ void store_row(float* base, int64_t i, const float* v
     for (int c = 0; c < L::QP / 4; ++c) p[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
 }
 __device__ __forceinline__ float4 ld4(const float* base, int64_t i, int qp, int c) {
-    return __ldg(reinterpret_cast<const float4*>(base + i * qp) + c);
+    return reinterpret_cast<const float4*>(base + i * qp)[c];
 }
 
 // The collision scratch S1, S1P of a scene of n nodes. D3Q27: node-major
@@ -162,18 +159,6 @@ __device__ __forceinline__ void s1_st(float* base, int64_t n, int64_t i, int c, 
         reinterpret_cast<float4*>(base + i * L::QP)[c] = v;
     }
 }
-// the whole row (slot order, QP floats of which the pads are not stored)
-template <class L>
-__device__ __forceinline__ void s1_store_row(float* base, int64_t n, int64_t i, const float* v) {
-    if constexpr (L::D == 2) {
-        float4* p = reinterpret_cast<float4*>(base + i * L::QS);
-#pragma unroll
-        for (int c = 0; c < L::NGATHER; ++c) p[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-        base[L::QS * n + i] = v[L::QS];
-    } else {
-        store_row<L>(base, i, v);
-    }
-}
 // neighbour-row gathers cached in L2 only (.cg): the rows of a pass's
 // neighbours are re-read by other passes long after L1 would have evicted
 // them, and allocating them in L1 costs more than it saves (D3Q27 RK gather:
@@ -185,13 +170,15 @@ __device__ __forceinline__ float4 ld4cg(const float* base, int64_t i, int qp, in
     return v;
 }
 // the gather load of a lattice: D3Q27 rows (112 B) bypass L1; D2Q9 rows
-// (48 B, 4.6x more nodes per line) keep the L1 reuse (measured both ways)
+// (48 B, 4.6x more nodes per line) keep the L1 reuse (measured both ways).
+// Plain loads, not ld.global.nc: a kernel may start before the one that writes
+// the rows has ended, so they are not read-only for its lifetime
 template <class L>
 __device__ __forceinline__ float4 ld4g(const float* base, int64_t i, int c) {
     if constexpr (L::D == 3)
         return ld4cg(base, i, L::QP, c);
     else
-        return __ldg(reinterpret_cast<const float4*>(base + i * L::QP) + c);
+        return reinterpret_cast<const float4*>(base + i * L::QP)[c];
 }
 // the same gather load on a stage or PML field row (L::QS floats)
 template <class L>
@@ -199,20 +186,17 @@ __device__ __forceinline__ float4 ld4s(const float* base, int64_t i, int c) {
     if constexpr (L::D == 3)
         return ld4cg(base, i, L::QS, c);
     else
-        return __ldg(reinterpret_cast<const float4*>(base + i * L::QS) + c);
+        return reinterpret_cast<const float4*>(base + i * L::QS)[c];
 }
 // the gather load of chunk c of a collision scratch row (s1_ld's layout)
 template <class L>
 __device__ __forceinline__ float4 s1_ldg(const float* base, int64_t n, int64_t j, int c) {
     if constexpr (L::D == 2) {
-        if (c >= L::NGATHER) return make_float4(__ldg(base + L::QS * n + j), 0.f, 0.f, 0.f);
-        return __ldg(reinterpret_cast<const float4*>(base + j * L::QS) + c);
+        if (c >= L::NGATHER) return make_float4(base[L::QS * n + j], 0.f, 0.f, 0.f);
+        return reinterpret_cast<const float4*>(base + j * L::QS)[c];
     } else {
         return ld4g<L>(base, j, c);
     }
-}
-__device__ __forceinline__ float4 ld4rw(const float* base, int64_t i, int qp, int c) {
-    return reinterpret_cast<const float4*>(base + i * qp)[c];
 }
 __device__ __forceinline__ void st4(float* base, int64_t i, int qp, int c, float4 v) {
     reinterpret_cast<float4*>(base + i * qp)[c] = v;
