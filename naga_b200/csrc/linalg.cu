@@ -47,28 +47,40 @@ __global__ void inverse_f64_kernel(const double* __restrict__ A, double* __restr
 // Register-resident Gauss-Jordan inverse of systems of up to 48 rows (the
 // stencil systems have n = k + D + 1: 19 / 20 for k = 16, 35 / 36 for k = 32).
 // N is the size the registers are laid out for: the system's own (n = N), or
-// with PAD the next of a few sizes, the rows and columns past n being those of
-// the identity, pivoted last. Lane l holds rows l and l + 32 in registers. Each elimination step publishes the scaled pivot
-// row in shared memory and every lane updates its rows from it, so the n^3
-// multiply-adds are independent register FMAs rather than a chain of
-// shared-memory read-modify-writes.
+// with PAD the next of a few sizes. Lane l holds rows l and l + 32 in
+// registers. Each elimination step publishes the pivot row in shared memory
+// and every lane updates its rows from it, so the n^3 multiply-adds are
+// independent register FMAs rather than a chain of shared-memory
+// read-modify-writes.
 //
 // Pivoting is virtual: every row carries its getrf position (the row order
 // after the swaps so far). The pivot of step k is the first row, in that
-// order, of maximal |a| among positions >= k. That is getrf's choice, so the
-// pivot sequence and info match the LU kernel. With B = P A the matrix in
+// order, of maximal |a| among positions k .. n - 1. That is getrf's choice, so
+// the pivot sequence and info match the LU kernel. With B = P A the matrix in
 // pivot order, the in-place sweep (pivot row scaled by p = 1 / a_kk, a_kk
 // replaced by p; every other row i: a_ij -= a_ik a_kj, a_ik = -a_ik p) leaves
 // row k of B^-1 in the row pivoted at step k. Since A^-1 = B^-1 P, the store
 // un-permutes: A^-1(k, r_m) = B^-1(k, m), with r_m the row pivoted at step m.
 //
 // Register columns rotate by one each step: at step k register j holds column
-// (k + j) mod n, so the pivot column is always register 0 and the new inverse
-// column enters at register n - 1; after n steps the order is the identity
-// again. The step loop therefore indexes no register by k.
+// (k + j) mod N, so the pivot column is always register 0 and the new inverse
+// column enters at register N - 1; after N steps the order is the identity
+// again, after n steps column c is in register c + N - n. The step loop
+// therefore indexes no register by k.
+//
+// PAD: n steps over n rows. The rows past n never leave position N, whatever
+// the values (a NaN or an infinity that a pivot row holds reaches them), so no
+// pivot and no store is ever one of theirs. The pivot row is published
+// unscaled and the rows are scaled by their reciprocal pivots at the end: the
+// multipliers a_ik p and the rows below the pivot are then the LU's own
+// values, with its range (a pivot row scaled first overflows where the
+// columns' scales differ by 1e155) and its exact zeros.
 //
 // Padded sizes against the LU in shared memory they had before: 100,000
-// systems of 24 x 24 2.24 -> 0.63 ms, 20,000 of 45 x 45 4.29 -> 0.87 ms.
+// systems of 24 x 24 2.20 -> 0.61 ms; 20,000 of 9 x 9 0.092 -> 0.045 ms, of
+// 33 x 33 2.02 -> 0.63, of 45 x 45 4.29 -> 0.84, of 48 x 48 5.75 -> 0.90; the
+// errors on RBF systems of 24 to 45 rows agree to 1 % (median 7.4e-15 both at
+// 24, 4.8e-13 at 45), info on singular integer matrices everywhere.
 // Measured alternatives, all slower or equal (10^6 systems of 36 x 36 on
 // B200, 18.6 ms for this form): per-row scales instead of rescaling the pivot
 // row (19.6 ms), the next pivot searched while the current step's columns
@@ -86,6 +98,7 @@ __global__ void __launch_bounds__(32 * kGjWarps, (N > 36 ? 4 : N > 32 ? 5 : 8))
                       int* __restrict__ info) {
     constexpr int S = (N + 31) / 32;
     constexpr int NP = (N + 1) & ~1;
+    static_assert(!PAD || N % 2 == 0, "a padded pivot row is published whole");
     const int n = PAD ? n_ : N;
     // per warp: the published pivot row (double-buffered by step parity) and
     // the physical row pivoted at each step
@@ -95,18 +108,19 @@ __global__ void __launch_bounds__(32 * kGjWarps, (N > 36 ? 4 : N > 32 ? 5 : 8))
     const int64_t nw = (int64_t)gridDim.x * kGjWarps;
     for (int64_t b = (int64_t)blockIdx.x * kGjWarps + w; b < batch; b += nw) {
         const double* ai = A + b * (int64_t)(n * n);
-        double a[S][N];
+        double a[S][N], scale[S];
         int pos[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             const int r = lane + 32 * s;
-            pos[s] = r < N ? r : N;  // N marks a padding row
+            pos[s] = r < n ? r : N;  // N marks a padding row
+            scale[s] = 0.0;
 #pragma unroll
-            for (int c = 0; c < N; ++c) a[s][c] = r < n && c < n ? ai[r + n * c] : (PAD && r == c ? 1.0 : 0.0);
+            for (int c = 0; c < N; ++c) a[s][c] = r < n && c < n ? ai[r + n * c] : 0.0;
         }
         int inf = 0;
 #pragma unroll 1
-        for (int k = 0; k < N; ++k) {
+        for (int k = 0; k < n; ++k) {
             // pivot: max |a| over positions >= k, ties to the lowest position.
             // |a| >= 0, so its bits order like unsigned integers.
             unsigned hi = 0, lo = 0;
@@ -133,49 +147,76 @@ __global__ void __launch_bounds__(32 * kGjWarps, (N > 36 ? 4 : N > 32 ? 5 : 8))
                 piv[s] = pos[s] == bpos;
                 pos[s] = pos[s] == k ? bpos : (piv[s] ? k : pos[s]);
             }
-            // the pivot row's owner scales it and publishes it rotated:
-            // pr[m] = a_r(m + 1) p for m < N - 1, pr[N - 1] = p
             double* pr = prow[w][k & 1];
-#pragma unroll
-            for (int s = 0; s < S; ++s)
-                if (piv[s]) {
-                    rowk[w][k] = lane + 32 * s;
-                    const double p = zero ? 0.0 : 1.0 / a[s][0];
-                    a[s][0] = p;
-#pragma unroll
-                    for (int j = 1; j < N; ++j) a[s][j] *= p;
-#pragma unroll
-                    for (int m = 0; m + 1 < N; m += 2)
-                        *reinterpret_cast<double2*>(pr + m) = make_double2(a[s][m + 1], m + 2 < N ? a[s][m + 2] : p);
-                    if (N & 1) pr[N - 1] = p;
-                }
-            __syncwarp();
-            // every row: a_i(m) = a_i(m + 1) - f_i pr[m] (rotated), the new
-            // column -f_i p; the pivot row (f = 0) only rotates, keeping p
             double f[S], l[S];
+            if constexpr (PAD) {
+                // published rotated: pr[m] = a_r(m + 1), the pivot last
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-                f[s] = piv[s] ? 0.0 : a[s][0];
-                l[s] = piv[s] ? a[s][0] : 0.0;
+                for (int s = 0; s < S; ++s)
+                    if (piv[s]) {
+                        rowk[w][k] = lane + 32 * s;
+#pragma unroll
+                        for (int m = 0; m < N; m += 2)
+                            *reinterpret_cast<double2*>(pr + m) = make_double2(a[s][m + 1], a[s][m + 2 < N ? m + 2 : 0]);
+                    }
+                __syncwarp();
+                // f_i = a_ik p, the new column -f_i; the pivot row (f = 0)
+                // takes 1 there. A zero pivot's reciprocal leaves NaN.
+                const double p = 1.0 / pr[N - 1];
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    f[s] = piv[s] ? 0.0 : a[s][0] * p;
+                    l[s] = piv[s] ? 1.0 : -f[s];
+                    if (piv[s]) scale[s] = p;
+                }
+            } else {
+                // the pivot row's owner scales it and publishes it rotated:
+                // pr[m] = a_r(m + 1) p for m < N - 1, pr[N - 1] = p
+#pragma unroll
+                for (int s = 0; s < S; ++s)
+                    if (piv[s]) {
+                        rowk[w][k] = lane + 32 * s;
+                        const double p = zero ? 0.0 : 1.0 / a[s][0];
+                        a[s][0] = p;
+#pragma unroll
+                        for (int j = 1; j < N; ++j) a[s][j] *= p;
+#pragma unroll
+                        for (int m = 0; m + 1 < N; m += 2)
+                            *reinterpret_cast<double2*>(pr + m) = make_double2(a[s][m + 1], m + 2 < N ? a[s][m + 2] : p);
+                        if (N & 1) pr[N - 1] = p;
+                    }
+                __syncwarp();
+                // the new column -f_i p; the pivot row (f = 0) only rotates,
+                // keeping p
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    f[s] = piv[s] ? 0.0 : a[s][0];
+                    l[s] = piv[s] ? a[s][0] : 0.0;
+                }
             }
+            // every row: a_i(m) = a_i(m + 1) - f_i pr[m] (rotated)
 #pragma unroll
             for (int m = 0; m < N; m += 2) {
                 const double2 q = *reinterpret_cast<const double2*>(pr + m);
 #pragma unroll
                 for (int s = 0; s < S; ++s) {
                     a[s][m] = fma(-f[s], q.x, m + 1 < N ? a[s][m + 1] : l[s]);
-                    if (m + 1 < N) a[s][m + 1] = fma(-f[s], q.y, m + 2 < N ? a[s][m + 2] : l[s]);
+                    if (PAD && m + 1 == N - 1)
+                        a[s][m + 1] = l[s];
+                    else if (m + 1 < N)
+                        a[s][m + 1] = fma(-f[s], q.y, m + 2 < N ? a[s][m + 2] : l[s]);
                 }
             }
         }
         __syncwarp();
         double* o = Ainv + b * (int64_t)(n * n);
+        const int c0 = N - n;  // register of column 0
 #pragma unroll
         for (int s = 0; s < S; ++s)
             if (lane + 32 * s < n)
 #pragma unroll
                 for (int j = 0; j < N; ++j)
-                    if (j < n) o[pos[s] + n * rowk[w][j]] = a[s][j];
+                    if (j >= c0) o[pos[s] + n * rowk[w][j - c0]] = PAD ? a[s][j] * scale[s] : a[s][j];
         if (info && lane == 0) info[b] = inf;
         __syncwarp();
     }

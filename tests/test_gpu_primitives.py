@@ -358,6 +358,54 @@ def test_inverse_nan_matrices_leave_the_batch_intact(naga, oracle, n):
     assert not np.isfinite(out[1]).any() and not np.isfinite(out[3]).all()
 
 
+@pytest.mark.parametrize("n", [7, 9, 23, 24, 33, 36, 45, 48, 49])
+def test_inverse_badly_scaled_systems_stay_in_place(naga, oracle, n):
+    """Systems whose elimination meets infinities (an infinite entry, a column
+    of subnormals, all entries subnormal) write nothing outside their own n x n
+    results: their neighbours are bit for bit what the batch gives without
+    them, and so is the memory past the last system, which is one of them."""
+    import torch
+
+    rng = np.random.default_rng(n + 7)
+    good = rng.standard_normal((10, n, n)) + 2 * np.eye(n)
+    A = good.copy()
+    A[1, 2, 4] = np.inf
+    A[3, n // 2] *= 1e-310
+    A[5] *= 1e-310
+    A[7, 1], A[7, 3] = A[7, 1] * 1e-155, A[7, 3] * 1e155
+    A[9, :, 1] = -np.inf
+
+    def run(a):
+        out = torch.full((a.size + 64 * 64,), -7.5, dtype=torch.float64, device="cuda")
+        src = _t(a)
+        assert naga.lib().naga_batched_inverse_f64(src.data_ptr(), out.data_ptr(), n, len(a), None,
+                                                   torch.cuda.current_stream().cuda_stream) == 0
+        out = _np(out)
+        assert (out[a.size:] == -7.5).all()
+        return out[: a.size].reshape(a.shape)
+
+    bad, ref = run(A), run(good)
+    for b in (0, 2, 4, 6, 8):
+        assert np.array_equal(bad[b], ref[b])
+
+
+@pytest.mark.parametrize("n", [7, 23, 33, 45, 49])
+def test_inverse_of_widely_scaled_columns(naga, oracle, n):
+    """Columns 400 decades apart do not meet in an LU (it only ever divides
+    within a column), so their inverse is as good as the unscaled system's:
+    row c of it is that one's over the column's scale."""
+    rng = np.random.default_rng(n + 8)
+    A = rng.standard_normal((5, n, n)) + 2 * np.eye(n)
+    scale = np.ones((5, n))
+    scale[:, 1], scale[:, n // 2] = 1e200, 1e-200
+    scale[3:, n - 1] = 1e-155
+    out, info = naga.batched_inverse_f64(_t(A * scale[:, :, None]))
+    assert (_np(info) == 0).all()
+    ref, _ = oracle.batched_inverse(A)
+    # element (c, r) of the inverse at [b, r, c]
+    _assert_inverse_close(_np(out) * scale[:, None, :], ref, A)
+
+
 @pytest.mark.parametrize("n", [19, 36])
 def test_inverse_register_sizes_singular_and_ties(naga, oracle, n):
     """The stencil sizes take the register Gauss-Jordan kernel: a zero
