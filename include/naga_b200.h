@@ -158,7 +158,8 @@ int naga_batched_inverse_f64(const double* A, double* A_inv, int n,
  * correction is below rel_tol relative to the column, or when the
  * correction stops shrinking (the FP64 residual's floor). info: as above,
  * or -1 when some column ended with a correction above both rel_tol and
- * 1e-10 of the column.                                                      */
+ * 1e-10 of the column, or is not finite (NaN or infinite entries, entries
+ * beyond FP32's range).                                                     */
 int naga_batched_inverse_f32r(const double* A, double* A_inv, int n,
                               int64_t batch, int max_iter, double rel_tol,
                               int* info, void* stream);

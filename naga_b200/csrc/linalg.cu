@@ -316,20 +316,23 @@ __device__ int warp_inverse_f32(const double* Af, int n, float* out, float* prow
 // of the shared-memory operands: 7 warps/SM (31 KB a system), a third of the
 // issue slots.
 // A column's refinement: last correction, the one before, and whether it is
-// done -- below the tolerance, or no longer contracting
+// done -- below the tolerance, no longer contracting, or not finite
 struct RefineState {
     double dlast = INFINITY, dprev = INFINITY, xlast = 0;
-    bool done;
+    bool done, lost = false;
     __device__ explicit RefineState(bool idle) : done(idle) {}
-    __device__ void update(float dm, double xm, double tol) {
+    // dm, xm: largest correction and entry (NaN not among them); finite:
+    // whether every correction is
+    __device__ void update(float dm, double xm, bool finite, double tol) {
         dprev = dlast;
         dlast = (double)dm;
         xlast = xm;
-        done = dlast <= tol * xm || dlast > 0.5 * dprev;
+        lost = !finite || !(xm < INFINITY);
+        done = lost || dlast <= tol * xm || dlast > 0.5 * dprev;
     }
     // last correction within the tolerance, or within 1e-10 of the column
     // when refinement stagnated at the FP64 residual floor
-    __device__ bool converged(double tol) const { return dlast <= tol * xlast || dlast <= 1e-10 * xlast; }
+    __device__ bool converged(double tol) const { return !lost && (dlast <= tol * xlast || dlast <= 1e-10 * xlast); }
 };
 template <int NP>
 struct RefineSize {
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(NP > 36 ? 128 : 224)
                     }
                 }
                 if (!st.done) {
-                    float dm = 0.f;
+                    float dm = 0.f, nil = 0.f;  // nil: NaN with any infinite or NaN correction
                     double xm = 0;
 #pragma unroll
                     for (int i = 0; i < NP; ++i) {
@@ -415,9 +418,10 @@ __global__ void __launch_bounds__(NP > 36 ? 128 : 224)
                         if (i < n) {
                             dm = fmaxf(dm, fabsf(d[i]));
                             xm = fmax(xm, fabs(x));
+                            nil = fmaf(d[i], 0.f, nil);
                         }
                     }
-                    st.update(dm, xm, tol);
+                    st.update(dm, xm, nil == 0.f, tol);
                 }
             }
             if (has) conv = st.converged(tol);
@@ -465,7 +469,7 @@ __global__ void __launch_bounds__(NP > 36 ? 128 : 224)
 #pragma unroll
                     for (int u = 0; u < RL; ++u) d[u] = fmaf(B[row[u] + NP * j], rj, d[u]);
                 }
-                float dm = 0.f;
+                float dm = 0.f, nil = 0.f;
                 double xm = 0;
 #pragma unroll
                 for (int u = 0; u < RL; ++u)
@@ -474,13 +478,15 @@ __global__ void __launch_bounds__(NP > 36 ? 128 : 224)
                         X[row[u] * NP + c] = x;
                         dm = fmaxf(dm, fabsf(d[u]));
                         xm = fmax(xm, fabs(x));
+                        nil = fmaf(d[u], 0.f, nil);
                     }
 #pragma unroll
                 for (int o = C; o < 32; o <<= 1) {
                     dm = fmaxf(dm, __shfl_xor_sync(kFull, dm, o));
                     xm = fmax(xm, __shfl_xor_sync(kFull, xm, o));
+                    nil += __shfl_xor_sync(kFull, nil, o);
                 }
-                if (!st.done) st.update(dm, xm, tol);
+                if (!st.done) st.update(dm, xm, nil == 0.f, tol);
                 __syncwarp();
             }
             if (has) conv = conv && st.converged(tol);

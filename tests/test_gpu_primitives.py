@@ -188,6 +188,24 @@ def test_inverse_every_register_size(naga, oracle, n):
     assert (err <= (4 + n) * np.finfo(np.float64).eps * np.linalg.cond(A)).all()
 
 
+@pytest.mark.parametrize("n", [7, 20, 33, 36, 45, 64])
+def test_inverse_refined_flags_what_is_not_finite(naga, oracle, n):
+    """NaN or infinite entries, and entries beyond FP32, are flagged -1 and
+    leave their neighbours alone."""
+    rng = np.random.default_rng(n + 9)
+    good = rng.standard_normal((7, n, n)) + 2 * np.eye(n)
+    A = good.copy()
+    A[1, 2, 4] = np.nan
+    A[2, n - 1, n - 1] = np.inf
+    A[4] *= 1e39
+    A[5] = np.nan
+    out, info = naga.batched_inverse_f32r(_t(A))
+    ref, rinfo = naga.batched_inverse_f32r(_t(good))
+    info = _np(info)
+    assert (info[[1, 2, 4, 5]] == -1).all() and (info[[0, 3, 6]] == 0).all() and (_np(rinfo) == 0).all()
+    assert np.array_equal(_np(out)[[0, 3, 6]], _np(ref)[[0, 3, 6]])
+
+
 def test_inverse_refined_flags_hopeless_systems(naga):
     """Condition ~1e12 is beyond FP32 refinement: flagged (-1), not silent."""
     rng = np.random.default_rng(1)
