@@ -153,8 +153,8 @@ int naga_knn_clouds(const float* pts, const int64_t* offsets, int n_clouds,
  * linalg/detail/batched_matrix_inverse.cuh:46-72). n <= 64.               */
 int naga_batched_inverse_f64(const double* A, double* A_inv, int n,
                              int64_t batch, int* info, void* stream);
-/* Same result computed from an FP32 LU with FP64-residual iterative
- * refinement of each column; a column stops at max_iter, when its
+/* Same result computed from an FP32 LU (its inverse where refinement
+ * converges fast) with FP64-residual iterative refinement of each column; a column stops at max_iter, when its
  * correction is below rel_tol relative to the column, or when the
  * correction stops shrinking (the FP64 residual's floor). info: as above,
  * or -1 when some column ended with a correction above both rel_tol and

@@ -1,7 +1,7 @@
 // Batched inverse of small dense matrices, one warp per matrix: FP64
 // Gauss-Jordan in registers for n <= 48 (the stencil systems among them), FP64
-// LU in shared memory for any other n <= 64, and FP32 factors with FP64
-// residual refinement.
+// LU in shared memory for any other n <= 64, and FP32 inverse or factors with
+// FP64 residual refinement.
 //
 // Replaces linalg::batched_matrix_inverse (linalg/batched_matrix_inverse.cuh:
 // 325-397), which hands slices of the batch to cuBLAS getrfBatched +
@@ -304,22 +304,98 @@ __device__ int warp_inverse_f32(const double* Af, int n, float* out, float* prow
     return inf > n ? 0 : inf;
 }
 
-// FP32 inverse, FP64 residual refinement of every column of the inverse:
-// X += B (I - A X) with B the FP32 inverse, one column a lane, 32 columns at
-// a time. The column's residual and correction accumulate in registers; A, B
-// and the column's own entries come from shared memory, A and B as broadcasts
-// shared by the warp's columns. A column is done when its correction falls
-// below the tolerance or no longer shrinks by half.
-// 20,000 systems of 36 x 36: 9.70 -> 1.30 ms, of 20 x 20 1.07 -> 0.27 ms, 5,000
-// of 45 x 45 6.27 -> 0.79 ms (before: triangular solves and residuals read and
-// written in shared memory, one dependent chain a lane). Bound by the latency
-// of the shared-memory operands: 7 warps/SM (31 KB a system), a third of the
-// issue slots.
+// FP32 LU of one system with getrf's pivoting, rows lane and lane + 32 of the
+// warp in registers; virtual pivoting and rotating columns as in
+// inverse_gj_kernel, the operations and their order those of warp_lu. Ad: the
+// FP64 system, column-major with stride NP; LU: its factors, the same layout,
+// rows in pivot order; rowk[i]: the row pivoted at step i; mult: NP x NP floats
+// for the multipliers by row as they arise (zeros stand in their place in the
+// registers, so the update passes over the eliminated columns); prow: NP
+// floats twice. Returns getrf's info; a zero pivot's column is left unreduced.
+template <int NP>
+__device__ int warp_lu_f32(const double* Ad, int n, float* LU, float* mult, float* prow, int* rowk) {
+    constexpr int S = (NP + 31) / 32;
+    const int lane = lane_id();
+    float a[S][NP];
+    int pos[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int r = lane + 32 * s;
+        pos[s] = r < n ? r : NP;  // NP: no row of the system, never a pivot
+#pragma unroll
+        for (int c = 0; c < NP; ++c) a[s][c] = r < n ? (float)Ad[r + NP * c] : 0.f;
+    }
+    int inf = 0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        unsigned h = 0u;
+        int bp = NP;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const unsigned v = __float_as_uint(a[s][0]) & 0x7fffffffu;
+            if (pos[s] >= k && pos[s] < NP && (v > h || (v == h && pos[s] < bp))) {
+                h = v;
+                bp = pos[s];
+            }
+        }
+        const unsigned m = __reduce_max_sync(kFull, h);
+        const int bpos = __reduce_min_sync(kFull, h == m ? bp : NP);
+        const bool zero = m == 0u;
+        if (zero && !inf) inf = k + 1;
+        float* const pr = prow + (k & 1) * NP;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const bool piv = pos[s] == bpos;
+            pos[s] = pos[s] == k ? bpos : (piv ? k : pos[s]);
+            if (piv) {
+                rowk[k] = lane + 32 * s;
+#pragma unroll
+                for (int c = 0; c < NP; c += 4)
+                    *reinterpret_cast<float4*>(pr + c) = make_float4(a[s][c], a[s][c + 1], a[s][c + 2], a[s][c + 3]);
+            }
+        }
+        __syncwarp();
+        const float inv = 1.f / pr[0];
+        float l[S], last[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const bool below = pos[s] > k && !zero;
+            l[s] = below ? a[s][0] * inv : 0.f;
+            last[s] = pos[s] > k ? 0.f : a[s][0];
+            if (lane + 32 * s < n) mult[lane + 32 * s + NP * k] = l[s];
+        }
+#pragma unroll
+        for (int c = 0; c < NP; c += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(pr + c);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                if (c > 0) a[s][c > 0 ? c - 1 : 0] = fmaf(-l[s], q.x, a[s][c]);
+                a[s][c] = fmaf(-l[s], q.y, a[s][c + 1]);
+                a[s][c + 1] = fmaf(-l[s], q.z, a[s][c + 2]);
+                a[s][c + 2] = fmaf(-l[s], q.w, a[s][c + 3]);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) a[s][NP - 1] = last[s];
+    }
+    __syncwarp();
+    const int c0 = NP - n;  // register of column 0
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+        if (lane + 32 * s < n)
+#pragma unroll
+            for (int c = 0; c < NP; ++c)
+                if (c >= c0)
+                    LU[pos[s] + NP * (c - c0)] = c - c0 < pos[s] ? mult[lane + 32 * s + NP * (c - c0)] : a[s][c];
+    __syncwarp();
+    return inf;
+}
+
 // A column's refinement: last correction, the one before, and whether it is
 // done -- below the tolerance, no longer contracting, or not finite
 struct RefineState {
     double dlast = INFINITY, dprev = INFINITY, xlast = 0;
-    bool done, lost = false;
+    bool done, lost = false, slow = false;
     __device__ explicit RefineState(bool idle) : done(idle) {}
     // dm, xm: largest correction and entry (NaN not among them); finite:
     // whether every correction is
@@ -329,53 +405,41 @@ struct RefineState {
         xlast = xm;
         lost = !finite || !(xm < INFINITY);
         done = lost || dlast <= tol * xm || dlast > 0.5 * dprev;
+        slow = slow || (dlast > dprev / 256 && dlast > 1e-10 * xm);
     }
     // last correction within the tolerance, or within 1e-10 of the column
     // when refinement stagnated at the FP64 residual floor
     __device__ bool converged(double tol) const { return !lost && (dlast <= tol * xlast || dlast <= 1e-10 * xlast); }
 };
-template <int NP>
-struct RefineSize {
-    static_assert(NP % 4 == 0, "16-B columns");
-    // A, X (FP64), B, R (FP32), the published rows and their order
-    static constexpr size_t per_warp = (size_t)NP * NP * (8 + 8 + 4 + 4) + NP * (8 + 4) + 32;
-    static constexpr size_t stride = (per_warp + 127) / 128 * 128;
-};
-template <int NP>
-__global__ void __launch_bounds__(NP > 36 ? 128 : 224)
-    inverse_f32r_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t batch, int max_iter,
-                        double tol, int* __restrict__ info, int warps_per_block) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int w = threadIdx.x >> 5, lane = lane_id();
-    double* Ad = reinterpret_cast<double*>(smem + RefineSize<NP>::stride * w);
-    double* X = Ad + NP * NP;  // X[j NP + c]: row j of column c
-    float* B = reinterpret_cast<float*>(X + NP * NP);
-    float* R = B + NP * NP;    // as X
-    float* prow = R + NP * NP;
-    int* rowk = reinterpret_cast<int*>(prow + 2 * NP);
-    const int64_t nw = (int64_t)gridDim.x * warps_per_block;
-    for (int64_t b = (int64_t)blockIdx.x * warps_per_block + w; b < batch; b += nw) {
-        const double* a = A + b * (int64_t)n * n;
-        for (int e = lane; e < NP * NP; e += 32) {
-            const int r = e % NP, c = e / NP;
-            Ad[e] = r < n && c < n ? a[r + (int64_t)n * c] : (r == c ? 1.0 : 0.0);
-        }
-        __syncwarp();
-        const int inf = warp_inverse_f32<NP>(Ad, n, B, prow, rowk);
-        bool conv = true;
-        // columns 0 .. 31, one a lane
-        {
-            const int c = lane;
-            const bool has = c < n;
-            const int cc = has ? c : 0;  // idle lanes read column 0
-            if (has)
-                for (int j = 0; j < NP; ++j) X[j * NP + c] = (double)B[j + NP * c];
-            RefineState st(!has);
-            for (int it = 0; it < max_iter && inf == 0 && !__all_sync(kFull, st.done); ++it) {
-                // residual R = I - A X
-                double r[NP];
+
+// FP64 residual refinement of every column of the inverse of one system, one
+// column a lane, 32 columns at a time. The column's residual and correction
+// stay in registers; A, the FP32 matrix M and the column's own entries come
+// from shared memory, A and M as broadcasts shared by the warp's columns.
+// FACTORS: M holds the factors of warp_lu_f32 and its corrections solve with
+// them (one straight run of code a column); X starts from 0. Otherwise M is the
+// FP32 inverse, X starts from it and a correction is its product with the
+// residual. True when every column of the lane converged -- with the inverse,
+// at 256 times a step down to 1e-10 of the column.
+template <int NP, bool FACTORS>
+__device__ bool refine(const double* Ad, const float* M, const int* rowk, double* X, float* R, int n, int max_iter,
+                       double tol) {
+    const int lane = lane_id();
+    bool conv = true;
+    // columns 0 .. 31, one a lane
+    {
+        const int c = lane;
+        const bool has = c < n;
+        const int cc = has ? c : 0;  // idle lanes read column 0
+        if (!FACTORS && has)
+            for (int j = 0; j < NP; ++j) X[j * NP + c] = (double)M[j + NP * c];
+        RefineState st(!has);
+        for (int it = FACTORS ? -1 : 0; it < 0 || (it < max_iter && !__all_sync(kFull, st.done)); ++it) {
+            // residual R = I - A X, to FP32
+            double r[NP];
 #pragma unroll
-                for (int i = 0; i < NP; ++i) r[i] = i == c ? 1.0 : 0.0;
+            for (int i = 0; i < NP; ++i) r[i] = i == c ? 1.0 : 0.0;
+            if (it >= 0) {
 #pragma unroll 2
                 for (int j = 0; j < n; ++j) {
                     const double xj = -X[j * NP + cc];
@@ -387,18 +451,51 @@ __global__ void __launch_bounds__(NP > 36 ? 128 : 224)
                         r[i + 1] = fma(v.y, xj, r[i + 1]);
                     }
                 }
-                if (has) {
+            }
+            if (has) {
 #pragma unroll
-                    for (int i = 0; i < NP; ++i) R[i * NP + c] = (float)r[i];
-                }
-                // correction D = B R, X += D
-                float d[NP];
+                for (int i = 0; i < NP; ++i) R[i * NP + c] = (float)r[i];
+            }
+            __syncwarp();
+            // correction D
+            float d[NP];
+            if constexpr (FACTORS) {
+#pragma unroll
+                for (int i = 0; i < NP; ++i) d[i] = i < n ? R[rowk[i] * NP + cc] : 0.f;
+#pragma unroll
+                for (int j = 0; j < NP; ++j)
+                    if (j < n) {
+                        const float4* col = reinterpret_cast<const float4*>(M + NP * j);
+#pragma unroll
+                        for (int i = (j + 1) / 4 * 4; i < NP; i += 4) {
+                            const float4 v = col[i / 4];
+                            if (i > j) d[i] = fmaf(-v.x, d[j], d[i]);
+                            if (i + 1 > j) d[i + 1] = fmaf(-v.y, d[j], d[i + 1]);
+                            if (i + 2 > j) d[i + 2] = fmaf(-v.z, d[j], d[i + 2]);
+                            if (i + 3 > j) d[i + 3] = fmaf(-v.w, d[j], d[i + 3]);
+                        }
+                    }
+#pragma unroll
+                for (int j = NP - 1; j >= 0; --j)
+                    if (j < n) {
+                        const float4* col = reinterpret_cast<const float4*>(M + NP * j);
+                        d[j] = d[j] / M[j + NP * j];
+#pragma unroll
+                        for (int i = 0; i < j; i += 4) {
+                            const float4 v = col[i / 4];
+                            d[i] = fmaf(-v.x, d[j], d[i]);
+                            if (i + 1 < j) d[i + 1] = fmaf(-v.y, d[j], d[i + 1]);
+                            if (i + 2 < j) d[i + 2] = fmaf(-v.z, d[j], d[i + 2]);
+                            if (i + 3 < j) d[i + 3] = fmaf(-v.w, d[j], d[i + 3]);
+                        }
+                    }
+            } else {
 #pragma unroll
                 for (int i = 0; i < NP; ++i) d[i] = 0.f;
 #pragma unroll 2
                 for (int j = 0; j < n; ++j) {
                     const float rj = R[j * NP + cc];
-                    const float4* col = reinterpret_cast<const float4*>(B + NP * j);
+                    const float4* col = reinterpret_cast<const float4*>(M + NP * j);
 #pragma unroll
                     for (int i = 0; i < NP; i += 4) {
                         const float4 v = col[i / 4];
@@ -408,94 +505,205 @@ __global__ void __launch_bounds__(NP > 36 ? 128 : 224)
                         d[i + 3] = fmaf(v.w, rj, d[i + 3]);
                     }
                 }
-                if (!st.done) {
-                    float dm = 0.f, nil = 0.f;  // nil: NaN with any infinite or NaN correction
-                    double xm = 0;
-#pragma unroll
-                    for (int i = 0; i < NP; ++i) {
-                        const double x = X[i * NP + c] + (double)d[i];
-                        X[i * NP + c] = x;
-                        if (i < n) {
-                            dm = fmaxf(dm, fabsf(d[i]));
-                            xm = fmax(xm, fabs(x));
-                            nil = fmaf(d[i], 0.f, nil);
-                        }
-                    }
-                    st.update(dm, xm, nil == 0.f, tol);
-                }
             }
-            if (has) conv = st.converged(tol);
-        }
-        __syncwarp();
-        // columns 32 .. n - 1, C at a time, 32 / C lanes a column: lane l
-        // takes rows (l / C) RL .. of column c0 + l % C, so the few columns
-        // past the lanes do not cost another full pass
-        constexpr int C = 4, RL = (NP + 32 / C - 1) / (32 / C);
-        for (int c0 = 32; c0 < n; c0 += C) {
-            const int c = c0 + lane % C, i0 = lane / C * RL;
-            const bool has = c < n;
-            const int cc = has ? c : c0;
-            if (has)
-                for (int u = 0; u < RL; ++u)
-                    if (i0 + u < NP) X[(i0 + u) * NP + c] = (double)B[i0 + u + NP * c];
-            __syncwarp();
-            RefineState st(!has);
-            for (int it = 0; it < max_iter && inf == 0 && !__all_sync(kFull, st.done); ++it) {
-                double r[RL];
-                float d[RL];
-                int row[RL];
+            // X += D
+            if (it < 0) {
+                if (has) {
 #pragma unroll
-                for (int u = 0; u < RL; ++u) {
-                    row[u] = i0 + u < NP ? i0 + u : NP - 1;
-                    r[u] = row[u] == c ? 1.0 : 0.0;
-                    d[u] = 0.f;
+                    for (int i = 0; i < NP; ++i) X[i * NP + c] = (double)d[i];
                 }
+            } else if (!st.done) {
+                float dm = 0.f, nil = 0.f;  // nil: NaN with any infinite or NaN correction
+                double xm = 0;
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    const double x = X[i * NP + c] + (double)d[i];
+                    X[i * NP + c] = x;
+                    if (i < n) {
+                        dm = fmaxf(dm, fabsf(d[i]));
+                        xm = fmax(xm, fabs(x));
+                        nil = fmaf(d[i], 0.f, nil);
+                    }
+                }
+                st.update(dm, xm, nil == 0.f, tol);
+            }
+            __syncwarp();
+        }
+        if (has) conv = st.converged(tol) && (FACTORS || !st.slow);
+    }
+    // columns 32 .. n - 1, C at a time, 32 / C lanes a column: lane l takes
+    // rows (l / C) RL .. of column c0 + l % C, so the few columns past the
+    // lanes do not cost another full pass
+    constexpr int C = 4, RL = (NP + 32 / C - 1) / (32 / C);
+    for (int c0 = 32; c0 < n; c0 += C) {
+        const int c = c0 + lane % C, i0 = lane / C * RL;
+        const bool has = c < n;
+        const int cc = has ? c : c0;
+        int row[RL];
+#pragma unroll
+        for (int u = 0; u < RL; ++u) row[u] = i0 + u < NP ? i0 + u : NP - 1;
+        if (!FACTORS && has)
+            for (int u = 0; u < RL; ++u)
+                if (i0 + u < NP) X[(i0 + u) * NP + c] = (double)M[i0 + u + NP * c];
+        __syncwarp();
+        RefineState st(!has);
+        for (int it = FACTORS ? -1 : 0; it < 0 || (it < max_iter && !__all_sync(kFull, st.done)); ++it) {
+            double r[RL];
+            float d[RL];
+#pragma unroll
+            for (int u = 0; u < RL; ++u) r[u] = row[u] == c ? 1.0 : 0.0;
+            if (it >= 0) {
 #pragma unroll 4
                 for (int j = 0; j < n; ++j) {
                     const double xj = -X[j * NP + cc];
 #pragma unroll
                     for (int u = 0; u < RL; ++u) r[u] = fma(Ad[row[u] + NP * j], xj, r[u]);
                 }
-                __syncwarp();
-                if (has) {
+            }
+            __syncwarp();
+            if (has) {
 #pragma unroll
-                    for (int u = 0; u < RL; ++u)
-                        if (i0 + u < NP) R[row[u] * NP + c] = (float)r[u];
-                }
-                __syncwarp();
+                for (int u = 0; u < RL; ++u)
+                    if (i0 + u < NP) R[row[u] * NP + c] = (float)r[u];
+            }
+            __syncwarp();
+            if constexpr (FACTORS) {
+                // x_j goes from its lane to the column's other lanes
+#pragma unroll
+                for (int u = 0; u < RL; ++u) d[u] = row[u] < n ? R[rowk[row[u]] * NP + cc] : 0.f;
+#pragma unroll 1
+                for (int o = 0; o < 32 / C; ++o)
+#pragma unroll
+                    for (int u = 0; u < RL; ++u) {
+                        const int j = o * RL + u;
+                        if (j >= n) continue;
+                        const float xj = __shfl_sync(kFull, d[u], o * C + lane % C);
+#pragma unroll
+                        for (int v = 0; v < RL; ++v)
+                            if (row[v] > j) d[v] = fmaf(-M[row[v] + NP * j], xj, d[v]);
+                    }
+#pragma unroll 1
+                for (int o = 32 / C - 1; o >= 0; --o)
+#pragma unroll
+                    for (int u = RL - 1; u >= 0; --u) {
+                        const int j = o * RL + u;
+                        if (j >= n) continue;
+                        const float xj = __shfl_sync(kFull, d[u], o * C + lane % C) / M[j + NP * j];
+                        if (lane / C == o) d[u] = xj;
+#pragma unroll
+                        for (int v = 0; v < RL; ++v)
+                            if (row[v] < j) d[v] = fmaf(-M[row[v] + NP * j], xj, d[v]);
+                    }
+            } else {
+#pragma unroll
+                for (int u = 0; u < RL; ++u) d[u] = 0.f;
 #pragma unroll 4
                 for (int j = 0; j < n; ++j) {
                     const float rj = R[j * NP + cc];
 #pragma unroll
-                    for (int u = 0; u < RL; ++u) d[u] = fmaf(B[row[u] + NP * j], rj, d[u]);
+                    for (int u = 0; u < RL; ++u) d[u] = fmaf(M[row[u] + NP * j], rj, d[u]);
                 }
-                float dm = 0.f, nil = 0.f;
-                double xm = 0;
-#pragma unroll
-                for (int u = 0; u < RL; ++u)
-                    if (!st.done && i0 + u < n) {
-                        const double x = X[row[u] * NP + c] + (double)d[u];
-                        X[row[u] * NP + c] = x;
-                        dm = fmaxf(dm, fabsf(d[u]));
-                        xm = fmax(xm, fabs(x));
-                        nil = fmaf(d[u], 0.f, nil);
-                    }
-#pragma unroll
-                for (int o = C; o < 32; o <<= 1) {
-                    dm = fmaxf(dm, __shfl_xor_sync(kFull, dm, o));
-                    xm = fmax(xm, __shfl_xor_sync(kFull, xm, o));
-                    nil += __shfl_xor_sync(kFull, nil, o);
-                }
-                if (!st.done) st.update(dm, xm, nil == 0.f, tol);
-                __syncwarp();
             }
-            if (has) conv = conv && st.converged(tol);
+            float dm = 0.f, nil = 0.f;
+            double xm = 0;
+#pragma unroll
+            for (int u = 0; u < RL; ++u)
+                if (!st.done && i0 + u < n) {
+                    const double x = (it < 0 ? 0.0 : X[row[u] * NP + c]) + (double)d[u];
+                    X[row[u] * NP + c] = x;
+                    dm = fmaxf(dm, fabsf(d[u]));
+                    xm = fmax(xm, fabs(x));
+                    nil = fmaf(d[u], 0.f, nil);
+                }
+#pragma unroll
+            for (int o = C; o < 32; o <<= 1) {
+                dm = fmaxf(dm, __shfl_xor_sync(kFull, dm, o));
+                xm = fmax(xm, __shfl_xor_sync(kFull, xm, o));
+                nil += __shfl_xor_sync(kFull, nil, o);
+            }
+            if (it >= 0 && !st.done) st.update(dm, xm, nil == 0.f, tol);
+            __syncwarp();
+        }
+        if (has) conv = conv && st.converged(tol) && (FACTORS || !st.slow);
+    }
+    __syncwarp();
+    return conv;
+}
+
+template <int NP>
+struct RefineSize {
+    static_assert(NP % 4 == 0, "16-B columns");
+    // A, X (FP64), M, R (FP32), the published rows and their order
+    static constexpr size_t per_warp = (size_t)NP * NP * (8 + 8 + 4 + 4) + NP * (8 + 4) + 32;
+    static constexpr size_t stride = (per_warp + 127) / 128 * 128;
+};
+
+// Refinement with the factors, for the systems the inverse does not serve.
+// Returns getrf's info, -1 when some column did not converge.
+template <int NP>
+__device__ __forceinline__ int refine_with_factors(const double* Ad, float* LU, double* X, float* R, float* prow, int* rowk,
+                                                int n, int max_iter, double tol) {
+    for (int e = lane_id(); e < NP * NP; e += 32) LU[e] = 0.f;
+    __syncwarp();
+    const int inf = warp_lu_f32<NP>(Ad, n, LU, R, prow, rowk);
+    const bool conv = refine<NP, true>(Ad, LU, rowk, X, R, n, inf ? 0 : max_iter, tol);
+    return inf ? inf : (__all_sync(kFull, conv) ? 0 : -1);
+}
+
+template <int NP>
+__device__ __noinline__ int refine_with_factors_call(const double* Ad, float* LU, double* X, float* R, float* prow,
+                                                     int* rowk, int n, int max_iter, double tol) {
+    return refine_with_factors<NP>(Ad, LU, X, R, prow, rowk, n, max_iter, tol);
+}
+
+// FP32 inverse or factors, FP64 residual refinement of every column of the
+// inverse. Most systems take the FP32 inverse: a correction is then one product
+// of independent multiply-adds. At the limit of what the refinement reaches
+// the inverse and the factors fail on different systems, about as often (of
+// 2000 systems of 2-D stencils with 32 supports, 50 and 41), so a system whose
+// corrections do not shrink 256 times a step is done again by solves with the
+// factors throughout, and the systems refused are those that these do not
+// reach: the same, over 30,000 systems of condition 1e6 and up, as with the
+// factors alone. (A bound of 16 reaches 3 to 70 % of those too, some with 1.6
+// times the error; 1024 sends random systems of 36 rows to the factors, 1.45 ->
+// 1.60 ms.)
+// Against triangular solves and residuals read and written in shared memory,
+// one dependent chain a lane: 20,000 systems of 36 x 36 9.70 -> 1.26 ms, of 20
+// x 20 1.08 -> 0.26; 5,000 of 45 x 45 8.1 -> 0.92, of 49 x 49 10.1 -> 2.5;
+// 3,000 of 64 x 64 18.0 -> 2.3 (solves with the factors for all of them:
+// 36 x 36 1.98, 45 x 45 2.5, 64 x 64 7.7). Bound by the latency of the
+// shared-memory operands: 7 warps/SM (31 KB a system), a third of the issue
+// slots. Up to 20 rows one warp a block: at 128 registers 14 fit an SM, and
+// small batches spread evenly (7 warps a block 0.28, 4 0.28 ms of 20 x 20).
+template <int NP>
+__global__ void __launch_bounds__(NP > 36 ? 128 : NP > 20 ? 224 : 32, NP > 20 ? 1 : 14)
+    inverse_f32r_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t batch, int max_iter,
+                        double tol, int* __restrict__ info, int warps_per_block) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int w = threadIdx.x >> 5, lane = lane_id();
+    double* Ad = reinterpret_cast<double*>(smem + RefineSize<NP>::stride * w);
+    double* X = Ad + NP * NP;  // X[j NP + c]: row j of column c
+    float* M = reinterpret_cast<float*>(X + NP * NP);
+    float* R = M + NP * NP;    // as X
+    float* prow = R + NP * NP;
+    int* rowk = reinterpret_cast<int*>(prow + 2 * NP);
+    const int64_t nw = (int64_t)gridDim.x * warps_per_block;
+    for (int64_t b = (int64_t)blockIdx.x * warps_per_block + w; b < batch; b += nw) {
+        const double* a = A + b * (int64_t)n * n;
+        for (int e = lane; e < NP * NP; e += 32) {
+            const int r = e % NP, c = e / NP;
+            Ad[e] = r < n && c < n ? a[r + (int64_t)n * c] : (r == c ? 1.0 : 0.0);
         }
         __syncwarp();
-        const bool ok = __all_sync(kFull, conv);
+        int inf = warp_inverse_f32<NP>(Ad, n, M, prow, rowk);
+        if (inf || !__all_sync(kFull, refine<NP, false>(Ad, M, rowk, X, R, n, max_iter, tol)))
+            // inlined where that keeps the path above from spilling around
+            // the call (5,000 of 45 x 45 0.96 -> 0.91 ms; 64 x 64 2.31 -> 2.39)
+            inf = NP == 48 ? refine_with_factors<NP>(Ad, M, X, R, prow, rowk, n, max_iter, tol)
+                           : refine_with_factors_call<NP>(Ad, M, X, R, prow, rowk, n, max_iter, tol);
         double* o = Ainv + b * (int64_t)n * n;
         for (int e = lane; e < n * n; e += 32) o[e] = X[(e % n) * NP + e / n];
-        if (info && lane == 0) info[b] = inf != 0 ? inf : (ok ? 0 : -1);
+        if (info && lane == 0) info[b] = inf;
         __syncwarp();
     }
 }
@@ -504,7 +712,7 @@ template <int NP>
 int launch_f32r(const double* A, double* Ainv, int n, int64_t batch, int max_iter, double tol, int* info,
                 cudaStream_t st) {
     const size_t stride = RefineSize<NP>::stride;
-    const int wpb = (int)std::min<size_t>(NP > 36 ? 4 : 7, smem_limit() / stride);
+    const int wpb = (int)std::min<size_t>(NP > 36 ? 4 : NP > 20 ? 7 : 1, smem_limit() / stride);
     if (wpb < 1) return set_error(NAGA_EINVAL, "batched inverse: matrix too large for shared memory");
     const size_t smem = stride * wpb;
     NAGA_CUDA_TRY(cudaFuncSetAttribute(inverse_f32r_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -150,7 +150,7 @@ def _assert_inverse_close(out, ref, A):
 @pytest.mark.parametrize("n", [3, 19, 20, 35, 36, 64])
 def test_inverse_matches_oracle(naga, oracle, n):
     rng = np.random.default_rng(n)
-    A = rng.standard_normal((300, n, n)) + 3 * np.eye(n)
+    A = rng.standard_normal((150, n, n)) + 3 * np.eye(n)
     out, info = naga.batched_inverse_f64(_t(A))
     ref, rinfo = oracle.batched_inverse(A)
     assert (_np(info) == 0).all()
@@ -186,6 +186,74 @@ def test_inverse_every_register_size(naga, oracle, n):
     assert (_np(info) == 0).all()
     err = np.abs(_np(out) - ref).max(axis=(1, 2)) / np.abs(ref).max(axis=(1, 2))
     assert (err <= (4 + n) * np.finfo(np.float64).eps * np.linalg.cond(A)).all()
+
+
+def _fma(a, b, c):
+    """a b + c rounded once: the exact product and sum as unevaluated pairs
+    (Dekker, Knuth), their tails added last."""
+    split = lambda x: (x * 134217729.0) - ((x * 134217729.0) - x)  # noqa: E731
+    a1, b1 = split(a), split(b)
+    a2, b2, p = a - a1, b - b1, a * b
+    pe = ((a1 * b1 - p) + a1 * b2 + a2 * b1) + a2 * b2
+    s = p + c
+    t = s - p
+    return s + (((p - (s - t)) + (c - t)) + pe)
+
+
+def _refined_by_factors(A, iters, tol=1e-14):
+    """Which systems of the batch an FP32 LU with FP64-residual refinement
+    leaves unconverged, every multiply-add rounded once and in the order of a
+    column sweep: at condition 1e6 and up it is the residual's rounding that
+    decides."""
+    f32 = np.float32
+    fma32 = lambda a, b, c: (a.astype(np.float64) * b + c).astype(f32)  # noqa: E731
+    m, n = A.shape[:2]
+    lu, perm, sys = A.astype(f32), np.tile(np.arange(n), (m, 1)), np.arange(m)
+    for j in range(n):
+        p = j + np.abs(lu[:, j:, j]).argmax(1)
+        for a in (lu, perm):
+            row = a[sys, p].copy()
+            a[sys, p] = a[:, j]
+            a[:, j] = row
+        lu[:, j + 1:, j] *= (f32(1) / lu[:, j, j])[:, None]
+        lu[:, j + 1:, j + 1:] = fma32(-lu[:, j + 1:, j, None], lu[:, j, None, j + 1:], lu[:, j + 1:, j + 1:])
+
+    def solve(r):
+        x = np.take_along_axis(r, perm[:, :, None], 1)
+        for j in range(n):
+            x[:, j + 1:] = fma32(-lu[:, j + 1:, j, None], x[:, j, None], x[:, j + 1:])
+        for j in reversed(range(n)):
+            x[:, j] /= lu[:, j, j, None]
+            x[:, :j] = fma32(-lu[:, :j, j, None], x[:, j, None], x[:, :j])
+        return x
+
+    eye = np.broadcast_to(np.eye(n), A.shape)
+    X = solve(eye.astype(f32)).astype(np.float64)
+    last, done = np.full((m, n), np.inf), np.zeros((m, n), bool)
+    for _ in range(iters):
+        r = eye.copy()
+        for j in range(n):
+            r = _fma(-A[:, :, j, None], X[:, j, None], r)
+        d = np.where(done[:, None], 0, solve(r.astype(f32)))
+        X = X + d
+        dm, xm = np.where(done, last, np.abs(d).max(1)), np.abs(X).max(1)
+        done = done | (dm <= tol * xm) | (dm > 0.5 * last)
+        last = dm
+    return ~((last <= tol * xm) | (last <= 1e-10 * xm)).all(1)
+
+
+@pytest.mark.parametrize("n,m,exponent", [(12, 300, 6.1), (35, 60, 5.85)])
+def test_inverse_refined_reaches_what_its_factors_reach(naga, n, m, exponent):
+    """Systems at the limit of FP32 refinement: exactly those that solves with
+    the FP32 factors leave unconverged are flagged, however the corrections
+    of others are computed."""
+    rng = np.random.default_rng(n)
+    q = lambda: np.linalg.qr(rng.standard_normal((m, n, n)))[0]  # noqa: E731
+    A = q() * np.where(np.arange(n) < n // 2, 1.0, 10.0 ** -exponent) @ q()
+    _, info = naga.batched_inverse_f32r(_t(A.transpose(0, 2, 1)), max_iter=20)
+    lost = _refined_by_factors(A, 20)
+    assert 0.1 * m < lost.sum() < 0.9 * m
+    assert np.array_equal(_np(info) != 0, lost), (_np(info).astype(bool) ^ lost).sum()
 
 
 @pytest.mark.parametrize("n", [7, 20, 33, 36, 45, 64])
