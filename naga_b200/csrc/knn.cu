@@ -431,7 +431,9 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
             const float T = (rad * w) * (rad * w);
             // the ball in cells, with room for the rounding of T, dist^2 and f
             const float rho = fmaf(rad, 1.f + 2e-5f, 1e-5f);
-            if (!(rho < 1e4f)) break;
+            // T beyond FP32: distances that overflow tie at infinity, and only
+            // the shell walk sees all of them
+            if (!(rho < 1e4f && T < INFINITY)) break;
             int a[3] = {0, 0, 0}, m[3] = {1, 1, 1};
 #pragma unroll
             for (int d = 1; d < D; ++d) {

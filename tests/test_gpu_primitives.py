@@ -62,10 +62,12 @@ def _awkward_cloud(kind, dim, rng):
         return np.stack(np.meshgrid(*[np.arange(m)] * dim, indexing="ij"), -1).reshape(-1, dim) / 16.0
     if kind == "far":  # large coordinates, coarse FP32 spacing
         return 1e5 + u(3000)
+    if kind == "vast":  # squared distances past a point's nearest few overflow FP32
+        return (u(3000) - 0.5) * 4e20
     return u(70)  # "few": barely more points than the largest k
 
 
-@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "lattice", "far", "few"])
+@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "lattice", "far", "vast", "few"])
 @pytest.mark.parametrize("dim,k", [(2, 16), (3, 32), (3, 33), (2, 64)])
 def test_knn_awkward_clouds(naga, oracle, kind, dim, k):
     """Self and free queries (inside, beside and far outside the cloud)
