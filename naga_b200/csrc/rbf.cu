@@ -558,13 +558,16 @@ __global__ void divergence_build_kernel(const float* __restrict__ pts, int64_t n
 // touched) from the scaled support coordinates xs. The RBF block by symmetry:
 // lane l evaluates the pairs (l, l + t mod KC), t = 0 .. KC / 2, and writes
 // both mirror entries to the assembly rows, of which it then reads its own.
+// shift, if given: a_l to take from row and column l of the RBF block.
 template <int D, int KC, int NR>
-__device__ __forceinline__ void assemble(GjSystem<KC, D, NR>& sys, const double* xs, int k, int shape, double* rows) {
+__device__ __forceinline__ void assemble(GjSystem<KC, D, NR>& sys, const double* xs, int k, int shape, double* rows,
+                                         const double* shift = nullptr) {
     using S = GjSystem<KC, D, NR>;
     const int l = lane_id();
     double xl[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) xl[d] = l < k ? xs[l * D + d] : 0.0;
+    const double al = shift && l < k ? shift[l] : 0.0;
     if (l < KC) {
 #pragma unroll 3
         for (int t = 0; t <= KC / 2; ++t) {
@@ -575,7 +578,11 @@ __device__ __forceinline__ void assemble(GjSystem<KC, D, NR>& sys, const double*
                 const double u = xl[d] - (c < k ? xs[c * D + d] : 0.0);
                 r2 += u * u;
             }
-            const double v = l < k && c < k ? shape_fn(r2, shape) : (l == c ? 1.0 : 0.0);
+            double v = l == c ? 1.0 : 0.0;
+            if (l < k && c < k) {
+                v = shape_fn(r2, shape);
+                if (shift) v -= al + shift[c];
+            }
             rows[l * S::LD + c] = v;
             rows[c * S::LD + l] = v;
         }
@@ -639,10 +646,12 @@ constexpr int kGjBlockWarps = 4;
 // Measured against the LU in shared memory that it replaces (every
 // multiply-add a shared-memory read-modify-write, 9 wavefronts per two columns
 // of a row): 250k nodes, k = 32: 8.6 -> 2.9 ms (100k nodes 3.7 -> 1.2 ms);
-// 50k weights 1.70 -> 0.45 ms. Bound by instruction issue at 16 warps/SM (128
+// 50k weights 1.70 -> 0.47 ms. Bound by instruction issue at 16 warps/SM (128
 // registers): half the issue slots, the FP64 pipe 28 % (the square roots of the
 // quadrature and the elimination in about equal parts). Relative error of the
-// FP64 weights against another FP64 solve: 1.1e-13, the LU 0.9e-13.
+// stencil's weights against 80-bit solves, mean over nodes: 3-D, k = 32,
+// multiquadric 5.8e-14, the LU 10.3e-14; 2-D, k = 16, cubic 1.42e-13, the LU
+// 1.51e-13.
 template <int D, int KC>
 __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
     divergence_build_gj_kernel(const float* __restrict__ pts, int64_t n, const uint32_t* __restrict__ idx, int k,
@@ -690,6 +699,17 @@ __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
 // Weights of up to NR queries of a group per solve (the elimination is run
 // again for every NR of them: the caller takes it for groups of at most NR).
 // T: type of the queries and the weights.
+//
+// The RBF block enters shifted, Phi_rc - a_r - a_c, and the right-hand sides
+// less a_r: the weights sum to 1 and the constant column takes up the rest, so
+// they are the same. With a_r = phi(|x_r - x|), x the first query, what is left
+// of a row is small, and the elimination of the polynomial columns rounds it
+// that much less (relative error of the weights in 3-D, k = 32, multiquadric:
+// 2.4e-15 unshifted, 1.7e-15 shifted, 1.9e-15 by an LU with the support columns
+// first; cubic in 2-D, k = 16: 1.13, 1.03 and 1.05e-14). A query outside its
+// support (nearer to none than 0.6 of the farthest) would make a_r the larger
+// part: x is then the nearest support (30 spacings off, cubic: 1.3e-12, the
+// LU 2.5e-12). a_r is rounded to FP32 so that the sum of two is exact.
 template <int D, int KC, int NR, class T>
 __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
     rbf_weights_gj_kernel(const float* __restrict__ src, int64_t nsrc, const uint32_t* __restrict__ support, int k,
@@ -703,7 +723,7 @@ __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
     double* rhs = pr + S::kRow;
     double* xs = rhs + S::kRhs;
     for (int64_t g = (int64_t)blockIdx.x * kGjBlockWarps + w; g < ngroups; g += (int64_t)gridDim.x * kGjBlockWarps) {
-        double o[D], xl[D];
+        double o[D], xl[D], r2o = 0;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
             o[d] = (double)qry[(g * group) * D + d];
@@ -719,11 +739,31 @@ __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
             for (int d = 0; d < D; ++d) {
                 xl[d] = ((double)src[(int64_t)j * D + d] - o[d]) / spacing;
                 xs[lane * D + d] = xl[d];
+                r2o += xl[d] * xl[d];
             }
         }
         __syncwarp();
+        // the shift's centre; squared distances compared by their upper words,
+        // the nearest support's lane in the low bits
+        const unsigned far = __reduce_max_sync(kFull, lane < k ? (unsigned)__double2hiint(0.36 * r2o) : 0u);
+        const unsigned near =
+            __reduce_min_sync(kFull, lane < k ? ((unsigned)__double2hiint(r2o) & ~31u) | (unsigned)lane : ~0u);
+        const double phi_o = shape_fn(r2o, shape);  // the first query is the origin
+        double c = phi_o;
+        if ((near & ~31u) > far) {
+            r2o = 0;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const double t = xl[d] - xs[(near & 31u) * D + d];
+                r2o += t * t;
+            }
+            c = shape_fn(r2o, shape);
+        }
+        const double al = (double)(float)c;
+        if (lane < k) pr[lane] = al;  // solve() publishes its rows there later
+        __syncwarp();
         S sys;
-        assemble<D, KC, NR>(sys, xs, k, shape, rows);
+        assemble<D, KC, NR>(sys, xs, k, shape, rows, pr);
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
             double x[D], r2 = 0;
@@ -733,7 +773,7 @@ __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
                 const double t = xl[d] - x[d];
                 r2 += t * t;
             }
-            sys.a[S::E + KC + q] = lane < k ? shape_fn(r2, shape) : 0.0;
+            sys.a[S::E + KC + q] = lane < k ? (q == 0 ? phi_o : shape_fn(r2, shape)) - al : 0.0;
             if (lane == 0) {
                 rhs[q] = 1.0;
 #pragma unroll

@@ -8,12 +8,15 @@
 // coefficients, which nobody asks for, so they are dropped and their lanes
 // take the constraint rows. The KC support columns follow over exactly KC
 // rows. This is LU with partial pivoting of the column-permuted system; no
-// second, nearly empty row per lane goes through the elimination.
+// second, nearly empty row per lane goes through the elimination. (It rounds
+// the RBF block at its full size E times more than an elimination that starts
+// with the support columns.)
 //
 // Step j: the pivot of column j is the row of largest |a| among the rows not
 // yet pivoted (magnitudes compared in their upper 15 bits of mantissa, by one
 // warp maximum over keys that carry the row's number; rows within that of each
-// other are equally good pivots). Its owner publishes it in shared memory and
+// other are equally good pivots: the error of the solution is the same to four
+// digits as with all bits compared). Its owner publishes it in shared memory and
 // every other row, pivoted ones too, subtracts its multiple: after the last
 // step row r holds b / pivot for the column it was pivoted on, with no back
 // substitution. Eliminating the pivoted rows costs no instruction: their lanes

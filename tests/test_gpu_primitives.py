@@ -310,6 +310,42 @@ def test_rbf_weights_every_padded_size(naga, oracle, dim, k, group):
     assert np.abs(w32 - ref).max() <= 1.2e-7 * scale
 
 
+@pytest.mark.parametrize("dim,k,group,off", [(2, 16, 1, 0), (3, 32, 1, 0), (3, 16, 4, 0), (2, 24, 1, 30), (3, 32, 1, 30)])
+def test_rbf_weights_round_no_more_than_an_lu(naga, dim, k, group, off):
+    """Error of the FP64 multiquadric weights against 80-bit solves, median
+    over 400 systems, beside LAPACK's LU of the same FP64 systems: queries
+    inside the support and `off` spacings outside. The bound, 1.1 of the LU's,
+    lies between the shifted system (0.9 and, outside, 0.05) and an
+    elimination that rounds the RBF block at its full size (1.3)."""
+    rng = np.random.default_rng(dim * 100 + k)
+    m = 400
+    X = rng.random((20 ** dim, dim)).astype(np.float32) * 20
+    centre = rng.random((m, dim)) * 14 + 3
+    near = np.argsort(((X[None] - centre[:, None]) ** 2).sum(-1), 1)[:, :k]
+    qry = centre[:, None] + rng.uniform(-0.2, 0.2, (m, group, dim)) + off * np.eye(dim)[0]
+    w = _np(naga.rbf_weights(_t(X), _t(near.astype(np.int32)), _t(qry.reshape(-1, dim)), group, 1.0, 0))
+
+    def system(t):
+        x = X[near].astype(t) - qry[:, :1].astype(t)
+        phi = lambda d: np.sqrt((d * d).sum(-1) + t(0.01))  # noqa: E731
+        A = np.zeros((m, k + dim + 1, k + dim + 1), t)
+        A[:, :k, :k] = phi(x[:, :, None] - x[:, None])
+        A[:, :k, k] = A[:, k, :k] = 1
+        A[:, :k, k + 1:], A[:, k + 1:, :k] = x, x.transpose(0, 2, 1)
+        q = qry.astype(t) - qry[:, :1].astype(t)
+        return A, np.concatenate([phi(x[:, :, None] - q[:, None]), np.ones((m, 1, group), t), q.transpose(0, 2, 1)], 1)
+
+    A, b = system(np.float64)
+    lu = np.linalg.solve(A, b)
+    A, b = system(np.longdouble)
+    ref = lu.astype(np.longdouble)
+    inv = np.linalg.inv(A.astype(np.float64)).astype(np.longdouble)
+    for _ in range(3):
+        ref = ref + np.einsum("bij,bjk->bik", inv, b - np.einsum("bij,bjk->bik", A, ref))
+    err = lambda y: np.median(np.linalg.norm(np.float64(y - ref[:, :k]), axis=1) / np.linalg.norm(np.float64(ref[:, :k]), axis=1))  # noqa: E731
+    assert err(w.reshape(m, group, k).transpose(0, 2, 1)) <= 1.1 * err(lu[:, :k])
+
+
 @pytest.mark.parametrize("dim,shape,precision", [(2, 0, 0), (2, 1, 0), (3, 0, 0), (3, 1, 0), (3, 1, 1)])
 def test_rbf_weights_match_oracle(naga, oracle, dim, shape, precision):
     rng = np.random.default_rng(dim * 10 + shape)
