@@ -884,6 +884,9 @@ extern "C" int naga_scene_destroy(naga_scene* s) {
     if (s->solo) naga_batch_destroy(s->solo);
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (void* p : s->allocs) cudaFreeAsync(p, s->stream);
+    // what the pool holds above its limit goes back to the system here, not
+    // at some later synchronisation of the process
+    if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->src_slot) cudaFree(s->src_slot);
     if (s->src_vals) cudaFree(s->src_vals);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -1388,6 +1391,7 @@ extern "C" int naga_batch_destroy(naga_batch* b) {
     if (!b->is_solo)
         for (auto* s : b->members) s->owner = nullptr;
     b->free_tables();
+    if (b->stream) cudaStreamSynchronize(b->stream);  // see naga_scene_destroy
     if (b->stream && !b->is_solo) cudaStreamDestroy(b->stream);
     delete b;
     return NAGA_OK;

@@ -338,6 +338,22 @@ def test_long_runs_equal_single_steps(naga, dim, n_side, layers):
     b.close()
 
 
+def test_destroyed_scenes_give_their_memory_back(naga):
+    """Closing scenes of 3 GB returns all but the 1 GB that the library's pool
+    may keep, without a further synchronisation."""
+    import torch
+
+    g = naga.generate_grid(3, 100, 4, 5)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    scenes = [naga.Scene(g, k=32, shape=0, probe_capacity=8) for _ in range(2)]
+    held = before - torch.cuda.mem_get_info()[0]
+    assert held > 2.2e9, held
+    for s in scenes:
+        s.close()
+    assert before - torch.cuda.mem_get_info()[0] < 1.15e9
+
+
 def test_async_probe_reads_match_synchronous(naga, oracle):
     """Probe samples queued every step behind the step (page-locked host
     buffer, one sync at the end) equal the synchronous read, including a
