@@ -408,10 +408,17 @@ int naga_batch_size(const naga_batch* batch);
 void* naga_batch_stream(naga_batch* batch);
 /* applies pending membership changes now: rebuilds the work lists, tunes
  * the launch shape of a new batch shape (naga_tuning_report) and captures
- * the step graph; naga_batch_step does the same when it is still pending.
- * Lets a caller keep that one-off work out of a timed window.            */
+ * the step graph and, unless the batch has only been stepped fewer than ten
+ * steps at a time, the graph of ten steps that long runs replay. Lets a
+ * caller keep that one-off work out of a timed window: after it no
+ * naga_batch_step captures a graph before the next membership change.     */
 int naga_batch_prepare(naga_batch* batch);
-/* enqueue nsteps steps of every member scene (asynchronous)              */
+/* enqueue nsteps steps of every member scene (asynchronous). Without
+ * naga_batch_prepare the one-off work happens here: at the first call after
+ * a membership change, and the ten-step graph (0.4 to 0.7 ms) at the call
+ * that brings the steps since then to 256. While a graph is being captured
+ * CUDA refuses a device-wide synchronisation by another thread. The same
+ * holds for naga_scene_step.                                             */
 int naga_batch_step(naga_batch* batch, int nsteps);
 int naga_batch_sync(naga_batch* batch);
 

@@ -148,6 +148,7 @@ struct naga_batch {
     cudaGraphExec_t exec = nullptr, run_exec = nullptr;
     int64_t replays = 0;     // steps replayed since the graph was captured
     bool run_tried = false;  // run_exec captured, or not to be had
+    int longest = 0;         // steps of the longest batch_step call yet
     // grow-only device tables (a membership change rewrites them in place on
     // the batch stream; they are reallocated only when they must grow)
     WorkItem* d_items = nullptr;  // the five item lists back to back
@@ -751,8 +752,7 @@ int capture_steps(naga_batch* b, int steps, cudaGraph_t* graph, cudaGraphExec_t*
 }
 
 // rebuilds the batch's item lists after a membership change, tunes the
-// launch shape of a new batch shape and captures the step graph, so that
-// the next batch_step only launches
+// launch shape of a new batch shape and captures the step graph
 int batch_prepare(naga_batch* b) {
     if (b->members.empty()) return NAGA_OK;
     int rc;
@@ -769,10 +769,24 @@ int batch_prepare(naga_batch* b) {
 // 10k in 3-D about 2 us less, 250k 480 -> 478 (4 steps a graph save two thirds
 // to all of it, 20 no more than 10).
 constexpr int kGraphSteps = 10;
-// Steps replayed one by one before that graph is captured: the capture takes
+// Steps of one membership from which that graph is captured: the capture takes
 // 0.4 to 0.7 ms, what it saves on about 250 steps, which a batch stepped a few
-// times between membership changes would not get back.
-constexpr int64_t kRunAfter = 128;
+// times between membership changes would not get back. Steps already replayed
+// and those of the call at hand count alike, so one long call on a fresh batch
+// takes the graph from its start.
+constexpr int64_t kRunAfter = 256;
+
+// captures the graph of long runs; without it (no memory for it, say) the
+// step graph goes on
+void batch_prepare_run(naga_batch* b) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+    b->run_tried = true;
+    if (capture_steps(b, kGraphSteps, &b->run_graph, &b->run_exec)) {
+        cudaGetLastError();
+        b->run_exec = nullptr;
+    }
+}
 
 int batch_step(naga_batch* b, int nsteps) {
     if (nsteps < 0) return set_error(NAGA_EINVAL, "step: negative step count");
@@ -785,21 +799,12 @@ int batch_step(naga_batch* b, int nsteps) {
             if ((rc = enqueue_step(b->dim, b->k, b->kb, P, b->stream))) return rc;
     } else {
         int left = nsteps;
-        if (!b->run_tried && b->replays >= kRunAfter && left >= kGraphSteps) {
-            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(b->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
-                b->run_tried = true;
-                // without it (no memory for it, say) the step graph goes on
-                if (capture_steps(b, kGraphSteps, &b->run_graph, &b->run_exec)) {
-                    cudaGetLastError();
-                    b->run_exec = nullptr;
-                }
-            }
-        }
+        if (!b->run_tried && b->replays + left >= kRunAfter && left >= kGraphSteps) batch_prepare_run(b);
         if (b->run_exec)
             for (; left >= kGraphSteps; left -= kGraphSteps) NAGA_CUDA_TRY(cudaGraphLaunch(b->run_exec, b->stream));
         for (; left > 0; --left) NAGA_CUDA_TRY(cudaGraphLaunch(b->exec, b->stream));
         b->replays += nsteps;
+        b->longest = std::max(b->longest, nsteps);
     }
     for (auto* s : b->members) s->steps += nsteps;
     return NAGA_OK;
@@ -1424,9 +1429,19 @@ extern "C" int naga_batch_remove(naga_batch* b, naga_scene* s) {
 extern "C" int naga_batch_size(const naga_batch* b) { return b ? (int)b->members.size() : 0; }
 extern "C" void* naga_batch_stream(naga_batch* b) { return b ? (void*)b->stream : nullptr; }
 
+int naga::batch_prepare_steps(naga_batch* b) { return batch_prepare(b); }
+
 extern "C" int naga_batch_prepare(naga_batch* b) {
     if (!b) return set_error(NAGA_EINVAL, "naga_batch_prepare: null batch");
-    return batch_prepare(b);
+    if (int rc = batch_prepare(b)) return rc;
+    // both graphs, so that no later step of this membership captures one; not
+    // the long runs' where the batch has only been stepped in short calls
+    // (a request loop that prepares after every membership change)
+    if (b->exec && !b->run_tried && !prof_on()) {
+        if (b->longest == 0 || b->longest >= kGraphSteps) batch_prepare_run(b);
+        b->run_tried = true;
+    }
+    return NAGA_OK;
 }
 
 extern "C" int naga_batch_step(naga_batch* b, int nsteps) {

@@ -26,4 +26,8 @@ struct GridScene {
 int build_grid_scene(const naga_grid_spec& spec, GridScene& out);
 int build_box_scene(const naga_box_grid_spec& spec, GridScene& out);
 
+// naga_batch_prepare for a caller that only steps singly: without the graph
+// of long runs
+int batch_prepare_steps(naga_batch* batch);
+
 }  // namespace naga

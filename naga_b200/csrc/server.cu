@@ -319,7 +319,7 @@ extern "C" int naga_server_tick(naga_server* s, int* n_active, int* n_queued) {
         const auto t0 = Clock::now();
         {
             std::lock_guard<std::mutex> cl(s->capture_mu);
-            rc = naga_batch_prepare(s->batch);
+            rc = batch_prepare_steps(s->batch);
         }
         if (rc) return rc;
         s->prepare_ms += ms_between(t0, Clock::now());

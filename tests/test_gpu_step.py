@@ -338,6 +338,49 @@ def test_long_runs_equal_single_steps(naga, dim, n_side, layers):
     b.close()
 
 
+def _runtime_calls(f):
+    """How often f makes each CUDA runtime call."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    return {n: names.count(n) for n in ("cudaGraphLaunch", "cudaStreamBeginCapture")}
+
+
+def test_long_runs_replay_ten_steps_a_graph(naga):
+    """One long call on a fresh scene replays graphs of ten steps from its
+    start, and leaves the state that single steps leave. After
+    naga_batch_prepare no step captures a graph, and the long runs' is there."""
+    g = naga.generate_grid(2, 25, 3, 5)
+    drho = naga.gaussian_pulse(g["points"], [0.5, 0.5], 1e-3, 0.08)
+    scenes = [naga.Scene(g, k=16, shape=1) for _ in range(4)]
+    for s in scenes:
+        s.set_density(drho)
+    long, single, batched, short = scenes
+    assert _runtime_calls(lambda: long.step(607)) == {"cudaGraphLaunch": 67, "cudaStreamBeginCapture": 2}
+    for _ in range(607):
+        single.step(1)
+    assert np.array_equal(long.state()[0], single.state()[0])
+    b = naga.Batch(2)
+    b.add(batched)
+    b.prepare()
+    assert _runtime_calls(lambda: [b.step(n) for n in (300, 1, 300, 6)]) == {"cudaGraphLaunch": 67,
+                                                                              "cudaStreamBeginCapture": 0}
+    assert np.array_equal(batched.state()[0], single.state()[0])
+    b.close()
+    # short calls, prepared after every change of members: one capture each
+    b = naga.Batch(2)
+    b.add(short)
+    b.step(1)
+    b.add(long)
+    assert _runtime_calls(b.prepare)["cudaStreamBeginCapture"] == 1
+    assert _runtime_calls(lambda: b.step(300)) == {"cudaGraphLaunch": 300, "cudaStreamBeginCapture": 0}
+    b.close()
+
+
 def test_destroyed_scenes_give_their_memory_back(naga):
     """Closing scenes of 3 GB returns all but the 1 GB that the library's pool
     may keep, without a further synchronisation."""
