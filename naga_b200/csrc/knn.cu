@@ -347,6 +347,68 @@ __device__ __noinline__ void query_shells(float x0, float x1, float x2, const Cl
     }
 }
 
+// Ranks of the first cnt (dist^2, index) keys among themselves; lane l holds
+// keys l, l + 32, ... By dist^2 alone, four comparisons a read; ranks that are
+// not all different (tied distances) are counted again with the index.
+// key has room for four entries past cnt.
+template <int PER>
+__device__ __forceinline__ void rank_keys(float* key, const unsigned* id, int cnt, float* mine, unsigned* who,
+                                          int* rank) {
+    const int lane = lane_id();
+    if (lane < 4) key[cnt + lane] = INFINITY;
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int e = lane + 32 * u;
+        mine[u] = e < cnt ? key[e] : INFINITY;
+        who[u] = e < cnt ? id[e] : 0xffffffffu;
+        rank[u] = 0;
+    }
+    for (int i = 0; i < cnt; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(key + i);
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            rank[u] += (v.x < mine[u]) + (v.y < mine[u]) + (v.z < mine[u]) + (v.w < mine[u]);
+    }
+    int distinct = 0;
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+        unsigned bits = 0;
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if (lane + 32 * u < cnt && rank[u] >> 5 == h) bits |= 1u << (rank[u] & 31);
+        distinct += __popc(__reduce_or_sync(kFull, bits));
+    }
+    if (distinct != cnt) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) rank[u] = 0;
+        for (int i = 0; i < cnt; ++i) {
+            const float kd = key[i];
+            const unsigned ki = id[i];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) rank[u] += cand_less(kd, ki, mine[u], who[u]);
+        }
+    }
+}
+
+// Keeps the k nearest of cnt >= k keys, in order; the k-th one's dist^2.
+template <int PER>
+__device__ __forceinline__ float keep_nearest(float* key, unsigned* id, int cnt, int k) {
+    float mine[PER];
+    unsigned who[PER];
+    int rank[PER];
+    rank_keys<PER>(key, id, cnt, mine, who, rank);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+        if (lane_id() + 32 * u < cnt && rank[u] < k) {
+            key[rank[u]] = mine[u];
+            id[rank[u]] = who[u];
+        }
+    __syncwarp();
+    return key[k - 1];
+}
+
 // Warp-per-query exact search by radius. R = 1 for k <= 32, 2 for k <= 64.
 //
 // The warp collects every point with dist^2 <= T in shared memory, T chosen
@@ -354,9 +416,11 @@ __device__ __noinline__ void query_shells(float x0, float x1, float x2, const Cl
 // index) keys against each other: the k of lowest rank are the answer, since
 // no point outside the collection is closer than one inside. T starts from
 // the cloud's mean density, corrected for the part of the ball outside the
-// bounding box, and is rescaled by the count found until k <= count <= CAP;
-// a query that does not settle in kTries rounds (clustered or tied points,
-// fewer points than k, a non-finite query) takes query_shells.
+// bounding box. Where more than CAP points turn up, the k nearest so far are
+// kept and T falls to the k-th one; a first ball whose rows hold far more is
+// shrunk before they are read. Where fewer than k turn up the ball grows. A
+// query that does not settle in kTries rounds or kRowsRead rows (an empty
+// neighbourhood, fewer points than k, a non-finite query) takes query_shells.
 //
 // The cells of the ball are walked by rows along x (one row a lane, clipped
 // to the ball), so a query reads ~2.5 k candidates instead of the ~8 k of
@@ -366,15 +430,25 @@ __device__ __noinline__ void query_shells(float x0, float x1, float x2, const Cl
 // same time within 10 %). Bound by instruction issue: ~1000 warp instructions
 // a query, 74 % of the issue slots, L1 38 %.
 //
+// Clouds of uneven density, 30,000 points, all as queries: coordinates cubed
+// from a normal distribution 1.9 ms at k = 32 and 2.2 at 64, a box with half of
+// its points in a thousandth of it 0.32 and 0.52 (with a ball that was searched
+// again wherever too many points turned up 3.5, 4.7, 0.58 and 0.66; shells of
+// cells with sorted insertion 1.9, 2.5, 0.66, 1.1).
+// At most 64 registers for k <= 32: 4 blocks/SM, 4.67 -> 4.36 ms on the 64
+// clouds.
+//
 // SELF: the queries are the sources; query q is the point at place q of the
 // cell order, so that a block's queries share cells.
-constexpr int kTries = 8;
+constexpr int kTries = 8, kRowsRead = 4096;
+constexpr int kShrinks = 2;      // rounds that may shrink the ball unread
+constexpr int kFarTooMany = 10;  // from this many times CAP points in its rows
 template <int R>
 struct QueryCap {
-    static constexpr int cap = 64 * R;  // keys collected at most
+    static constexpr int cap = 64 * R;  // keys collected at most: 32 R to keep, and a warp's more
 };
 template <int D, int R, bool SELF>
-__global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq, const int64_t* q_offsets,
+__global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float* qry, int64_t nq, const int64_t* q_offsets,
                                                     int q_nclouds, const CloudGrid* grids,
                                                     const unsigned* cell_start, const float4* sorted,
                                                     int k, uint32_t* out_idx, float* out_d2) {
@@ -425,10 +499,10 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
         }
         // radius in cells; past the box, the distance to it comes on top
         float rad = fmaf(r0, exp2f((-1.f / D) * __log2f(inside)), sqrtf(out2));
-        float rad_lo = 0.f, rad_hi = INFINITY;  // counts below k / above CAP
+        int rows_read = 0;
         bool done = false;
         for (int tries = 0; ok && tries < kTries; ++tries) {
-            const float T = (rad * w) * (rad * w);
+            float T = (rad * w) * (rad * w);
             // the ball in cells, with room for the rounding of T, dist^2 and f
             const float rho = fmaf(rad, 1.f + 2e-5f, 1e-5f);
             // T beyond FP32: distances that overflow tie at infinity, and only
@@ -443,9 +517,12 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
                 m[d] = hi - lo + 1;
             }
             const int nrows = m[1] > 0 && m[2] > 0 ? m[1] * m[2] : 0;
-            if (nrows > 1024) break;
+            rows_read += nrows;
+            if (nrows > 1024 || rows_read > kRowsRead) break;
             int cnt = 0;
-            for (int t0 = 0; t0 < nrows && cnt <= 2 * CAP; t0 += 32) {
+            unsigned seen = 0;  // points of the rows read
+            bool shrink = false;
+            for (int t0 = 0; t0 < nrows; t0 += 32) {
                 unsigned sb = 0, len = 0;
                 const int t = t0 + lane;
                 if (t < nrows) {
@@ -479,13 +556,16 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
                     if (lane >= o) incl += v;
                 }
                 const unsigned excl = incl - len, total = __shfl_sync(kFull, incl, 31);
+                seen += total;
+                shrink = seen > kFarTooMany * CAP && tries < kShrinks;
+                if (shrink) break;
                 // the non-empty rows in order: item i of the chunk is point
                 // row_off[rank of its row] + i
                 const unsigned some = __ballot_sync(kFull, len > 0);
                 if (len > 0) row_off[__popc(some & below)] = sb - excl;
                 __syncwarp();
                 int before = 0;  // rows begun in earlier batches
-                for (unsigned base = 0; base < total && cnt <= 2 * CAP; base += 32) {
+                for (unsigned base = 0; base < total; base += 32) {
                     const bool head = len > 0 && excl - base < 32u;
                     const unsigned heads = __reduce_or_sync(kFull, head ? 1u << (excl - base) : 0u);
                     const unsigned i = base + lane;
@@ -499,10 +579,15 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
                         cd = dist2_ref<D>(x, sv);
                         ci = __float_as_uint(s.w);
                     }
-                    const bool take = cd <= T;
-                    const unsigned mask = __ballot_sync(kFull, take);
-                    const int pos = cnt + __popc(mask & below);
-                    if (take && pos < CAP) {
+                    unsigned mask = __ballot_sync(kFull, cd <= T);
+                    if (cnt + __popc(mask) > CAP) {
+                        __syncwarp();
+                        T = keep_nearest<PER>(key, id, cnt, k);
+                        cnt = k;
+                        mask = __ballot_sync(kFull, cd <= T);
+                    }
+                    if (cd <= T) {
+                        const int pos = cnt + __popc(mask & below);
                         key[pos] = cd;
                         id[pos] = ci;
                     }
@@ -510,47 +595,11 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
                 }
                 __syncwarp();
             }
-            if (cnt >= k && cnt <= CAP) {
-                // rank the keys (lane l holds keys l, l + 32, ...) by dist^2
-                // alone, four comparisons a read; ranks that are not all
-                // different (tied distances) are counted again with the index
-                if (lane < 4) key[cnt + lane] = INFINITY;
-                __syncwarp();
+            if (!shrink && cnt >= k) {
                 float mine[PER];
                 unsigned who[PER];
                 int rank[PER];
-#pragma unroll
-                for (int u = 0; u < PER; ++u) {
-                    const int e = lane + 32 * u;
-                    mine[u] = e < cnt ? key[e] : INFINITY;
-                    who[u] = e < cnt ? id[e] : 0xffffffffu;
-                    rank[u] = 0;
-                }
-                for (int i = 0; i < cnt; i += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(key + i);
-#pragma unroll
-                    for (int u = 0; u < PER; ++u)
-                        rank[u] += (v.x < mine[u]) + (v.y < mine[u]) + (v.z < mine[u]) + (v.w < mine[u]);
-                }
-                int distinct = 0;
-#pragma unroll
-                for (int h = 0; h < PER; ++h) {
-                    unsigned bits = 0;
-#pragma unroll
-                    for (int u = 0; u < PER; ++u)
-                        if (lane + 32 * u < cnt && rank[u] >> 5 == h) bits |= 1u << (rank[u] & 31);
-                    distinct += __popc(__reduce_or_sync(kFull, bits));
-                }
-                if (distinct != cnt) {
-#pragma unroll
-                    for (int u = 0; u < PER; ++u) rank[u] = 0;
-                    for (int i = 0; i < cnt; ++i) {
-                        const float kd = key[i];
-                        const unsigned ki = id[i];
-#pragma unroll
-                        for (int u = 0; u < PER; ++u) rank[u] += cand_less(kd, ki, mine[u], who[u]);
-                    }
-                }
+                rank_keys<PER>(key, id, cnt, mine, who, rank);
 #pragma unroll
                 for (int u = 0; u < PER; ++u)
                     if (lane + 32 * u < cnt && rank[u] < k) {
@@ -562,18 +611,11 @@ __global__ void __launch_bounds__(256) query_kernel(const float* qry, int64_t nq
                 break;
             }
             __syncwarp();
-            // rescale towards 1.4 k points, inside the bracket
-            if (cnt < k) {
-                rad_lo = rad;
-                const float s = 1.4f * (float)k / fmaxf((float)cnt, 1.f);
-                rad *= fminf(3.f, fmaxf(1.05f, D == 2 ? sqrtf(s) : cbrtf(s)));
-                if (rad >= rad_hi) rad = 0.5f * (rad_lo + rad_hi);
-            } else {
-                rad_hi = rad;
-                const float s = 1.4f * (float)k / (float)cnt;
-                rad *= D == 2 ? sqrtf(s) : cbrtf(s);
-                if (rad <= rad_lo) rad = 0.5f * (rad_lo + rad_hi);
-            }
+            // to 1.4 k points by the count found, to 8 k or so by the rows' points
+            // (two fifths of them lie in the ball)
+            const float s = (float)k * (shrink ? 20.f / (float)seen : 1.4f / fmaxf((float)cnt, 1.f));
+            const float step = D == 2 ? sqrtf(s) : cbrtf(s);
+            rad *= shrink ? step : fminf(2.f, fmaxf(1.05f, step));
         }
         if (!done)
             query_shells<D, R>(x[0], x[1], x[2], grids + cl, cell_start, sorted, k, out_idx + q * k, out_d2 + q * k);

@@ -60,6 +60,13 @@ def _awkward_cloud(kind, dim, rng):
     if kind == "lattice":  # exact distance ties at every radius
         m = 14 if dim == 3 else 50
         return np.stack(np.meshgrid(*[np.arange(m)] * dim, indexing="ij"), -1).reshape(-1, dim) / 16.0
+    if kind == "spike":  # density without bound at the centre
+        return rng.standard_normal((4000, dim)) ** 3
+    if kind == "corner":  # half of the points in a thousandth of the box
+        return np.concatenate([u(2000), u(2000) * 0.1])
+    if kind == "shell":  # nothing inside
+        p = rng.standard_normal((4000, dim))
+        return p / np.linalg.norm(p, axis=1, keepdims=True)
     if kind == "far":  # large coordinates, coarse FP32 spacing
         return 1e5 + u(3000)
     if kind == "vast":  # squared distances past a point's nearest few overflow FP32
@@ -67,8 +74,9 @@ def _awkward_cloud(kind, dim, rng):
     return u(70)  # "few": barely more points than the largest k
 
 
-@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "lattice", "far", "vast", "few"])
-@pytest.mark.parametrize("dim,k", [(2, 16), (3, 32), (3, 33), (2, 64)])
+@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "lattice", "spike", "corner", "shell", "far", "vast",
+                                  "few"])
+@pytest.mark.parametrize("dim,k", [(2, 16), (3, 32), (3, 33), (2, 64), (3, 1)])
 def test_knn_awkward_clouds(naga, oracle, kind, dim, k):
     """Self and free queries (inside, beside and far outside the cloud)
     against the oracle, bit for bit: the radius search, its rescaling, and
