@@ -675,8 +675,11 @@ __device__ __noinline__ int refine_with_factors_call(const double* Ad, float* LU
 // shared-memory operands: 7 warps/SM (31 KB a system), a third of the issue
 // slots. Up to 20 rows one warp a block: at 128 registers 14 fit an SM, and
 // small batches spread evenly (7 warps a block 0.28, 4 0.28 ms of 20 x 20).
+// Up to 8 and 4 rows registers of their own, or the smallest systems would be
+// slower than by a chain a lane: 20,000 of 2 x 2 0.047 (by chains) and 0.129
+// (padded to 20) -> 0.032 ms, of 8 x 8 0.22 and 0.18 -> 0.073.
 template <int NP>
-__global__ void __launch_bounds__(NP > 36 ? 128 : NP > 20 ? 224 : 32, NP > 20 ? 1 : 14)
+__global__ void __launch_bounds__(NP > 36 ? 128 : NP > 20 ? 224 : 32, NP > 20 ? 1 : NP > 8 ? 14 : 24)
     inverse_f32r_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t batch, int max_iter,
                         double tol, int* __restrict__ info, int warps_per_block) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -763,6 +766,8 @@ int batched_inverse(const double* A, double* Ainv, int n, int64_t batch, int* in
         return launch_gj<48, true>(A, Ainv, n, batch, info, st);
     }
     if (refined) {
+        if (n <= 4) return launch_f32r<4>(A, Ainv, n, batch, max_iter, tol, info, st);
+        if (n <= 8) return launch_f32r<8>(A, Ainv, n, batch, max_iter, tol, info, st);
         if (n <= 20) return launch_f32r<20>(A, Ainv, n, batch, max_iter, tol, info, st);
         if (n <= 28) return launch_f32r<28>(A, Ainv, n, batch, max_iter, tol, info, st);
         if (n <= 36) return launch_f32r<36>(A, Ainv, n, batch, max_iter, tol, info, st);
