@@ -417,8 +417,9 @@ __device__ __forceinline__ float keep_nearest(float* key, unsigned* id, int cnt,
 // no point outside the collection is closer than one inside. T starts from
 // the cloud's mean density, corrected for the part of the ball outside the
 // bounding box. Where more than CAP points turn up, the k nearest so far are
-// kept and T falls to the k-th one; a first ball whose rows hold far more is
-// shrunk before they are read. Where fewer than k turn up the ball grows. A
+// kept and T falls to the k-th one; a ball whose rows hold far more is shrunk
+// before they are read (the first ones, and one that grew well past a radius
+// with too few). Where fewer than k turn up the ball grows. A
 // query that does not settle in kTries rounds or kRowsRead rows (an empty
 // neighbourhood, fewer points than k, a non-finite query) takes query_shells.
 //
@@ -441,7 +442,7 @@ __device__ __forceinline__ float keep_nearest(float* key, unsigned* id, int cnt,
 // SELF: the queries are the sources; query q is the point at place q of the
 // cell order, so that a block's queries share cells.
 constexpr int kTries = 8, kRowsRead = 4096;
-constexpr int kShrinks = 2;      // rounds that may shrink the ball unread
+constexpr int kShrinks = 2;      // first rounds that may shrink the ball unread
 constexpr int kFarTooMany = 10;  // from this many times CAP points in its rows
 template <int R>
 struct QueryCap {
@@ -499,6 +500,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float*
         }
         // radius in cells; past the box, the distance to it comes on top
         float rad = fmaf(r0, exp2f((-1.f / D) * __log2f(inside)), sqrtf(out2));
+        float rad_lo = 0.f;  // the largest radius with too few
         int rows_read = 0;
         bool done = false;
         for (int tries = 0; ok && tries < kTries; ++tries) {
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float*
                 }
                 const unsigned excl = incl - len, total = __shfl_sync(kFull, incl, 31);
                 seen += total;
-                shrink = seen > kFarTooMany * CAP && tries < kShrinks;
+                shrink = seen > kFarTooMany * CAP && (tries < kShrinks || (rad_lo > 0.f && rad_lo < 0.6f * rad));
                 if (shrink) break;
                 // the non-empty rows in order: item i of the chunk is point
                 // row_off[rank of its row] + i
@@ -612,10 +614,12 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float*
             }
             __syncwarp();
             // to 1.4 k points by the count found, to 8 k or so by the rows' points
-            // (two fifths of them lie in the ball)
+            // (two fifths of them lie in the ball), halfway to a radius with
+            // too few
             const float s = (float)k * (shrink ? 20.f / (float)seen : 1.4f / fmaxf((float)cnt, 1.f));
             const float step = D == 2 ? sqrtf(s) : cbrtf(s);
-            rad *= shrink ? step : fminf(2.f, fmaxf(1.05f, step));
+            if (!shrink) rad_lo = rad;
+            rad = shrink ? fmaxf(rad * step, sqrtf(rad * rad_lo)) : rad * fminf(2.f, fmaxf(1.05f, step));
         }
         if (!done)
             query_shells<D, R>(x[0], x[1], x[2], grids + cl, cell_start, sorted, k, out_idx + q * k, out_d2 + q * k);
