@@ -87,8 +87,9 @@ struct naga_server {
     int64_t done = 0, failed = 0;   // mu
     std::mutex mu;
     // held around the batch's graph capture (tick thread) and around the
-    // set-up thread's frees: cudaFree synchronises the device, which a
-    // stream capture in progress must not see
+    // set-up thread's frees: a scene's buffers go back to the pool on its own
+    // stream, but its source arrays by cudaFree, which synchronises the device,
+    // and that a stream capture in progress must not see
     std::mutex capture_mu;
     std::condition_variable cv;
     bool stop = false;

@@ -426,7 +426,6 @@ __device__ __forceinline__ void collide(const float* g, float drho, const float*
 }
 
 // ------------------------------------------------------------- kernels
-// SceneDev of the current item into shared memory (warp 0 copies words)
 // Programmatic dependent launch between the step's kernels: a kernel lets
 // the next one be scheduled once all its blocks have finished their work
 // (earlier, the waiting blocks of later kernels took SM slots from the
@@ -446,11 +445,13 @@ __device__ __forceinline__ void pdl_wait_prev() { asm volatile("griddepcontrol.w
 // boundary kernels). Up to 148 blocks gave the same, up to 296 a step of 10k
 // nodes in 3-D 50 -> 54 us, and two such scenes on streams of their own lost
 // 3 % at 148, 18 % at 296: the waiting blocks of one keep the other's out.
-constexpr unsigned kFewBlocks = 74;
+constexpr unsigned kSms = 148;  // of a B200, the one device the code is built for
+constexpr unsigned kFewBlocks = kSms / 2;
 __device__ __forceinline__ void pdl_allow_next_if_few() {
     if (gridDim.x * gridDim.y <= kFewBlocks) pdl_allow_next();
 }
 
+// SceneDev of the current item into shared memory (warp 0 copies words)
 __device__ __forceinline__ void load_scene(SceneDev& dst, const SceneDev* src) {
     if (threadIdx.x < 32) {
         const int* a = reinterpret_cast<const int*>(src);

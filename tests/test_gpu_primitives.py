@@ -450,33 +450,40 @@ def test_knn_clouds_ragged(naga, oracle):
         assert np.array_equal(d2[off[c]:off[c + 1]], od)
 
 
-def test_inverse_singular_and_empty(naga, oracle):
+@pytest.mark.parametrize("n", [9, 23, 36, 45, 49, 64])
+def test_inverse_singular_and_empty(naga, oracle, n):
     """A matrix with an exactly zero column reports the LAPACK info (the
-    1-based column of the zero pivot) like the oracle; its neighbours in
-    the batch are unaffected; an empty batch is a no-op."""
+    1-based column of the zero pivot) like the oracle, on the padded (9, 23,
+    45) and the exact (36) register kernel and on the shared-memory LU (49,
+    64), and a matrix with two equal columns of small integers, which every
+    elimination cancels exactly, a zero pivot; their neighbours in the batch
+    are unaffected; an empty batch is a no-op."""
     import torch
 
     rng = np.random.default_rng(3)
-    n = 9
     A = rng.standard_normal((6, n, n)) + 3 * np.eye(n)
     A[2, 4, :] = 0.0  # column 5 of matrix 2 (element (i, j) at A[b, j, i])
+    A[4] = np.eye(n)
+    A[4, n - 1] = A[4, 3] + A[4, 4]
+    A[4, 2] = A[4, n - 1]
     out, info = naga.batched_inverse_f64(_t(A))
     ref, rinfo = oracle.batched_inverse(A)
     info = _np(info)
     assert info[2] == rinfo[2] and info[2] > 0
-    ok = [b for b in range(6) if b != 2]
+    assert info[4] == rinfo[4] and info[4] > 0
+    ok = [0, 1, 3, 5]
     assert (info[ok] == 0).all()
-    assert np.abs(_np(out)[ok] - ref[ok]).max() / np.abs(ref[ok]).max() < 1e-12
+    _assert_inverse_close(_np(out)[ok], ref[ok], A[ok])
     out0, info0 = naga.batched_inverse_f64(torch.empty((0, n, n), dtype=torch.float64, device="cuda"))
     assert tuple(out0.shape) == (0, n, n) and tuple(info0.shape) == (0,)
 
 
-@pytest.mark.parametrize("n", [9, 36])
+@pytest.mark.parametrize("n", [9, 23, 36, 45, 49, 64])
 def test_inverse_nan_matrices_leave_the_batch_intact(naga, oracle, n):
     """Matrices with NaN entries (all of them, or one) in the middle of a
     batch: their results are not finite and their neighbours still match
-    the oracle, on the shared-memory LU (n = 9) and the register
-    Gauss-Jordan kernel (n = 36)."""
+    the oracle, on the padded (9, 23, 45) and the exact (36) register
+    Gauss-Jordan kernel and on the shared-memory LU (49, 64)."""
     rng = np.random.default_rng(n + 1)
     A = rng.standard_normal((5, n, n)) + 3 * np.eye(n)
     A[1] = np.nan
