@@ -409,59 +409,226 @@ __device__ __forceinline__ float keep_nearest(float* key, unsigned* id, int cnt,
     return key[k - 1];
 }
 
+// a query in cells of its cloud's grid: cell c0 and the place f in [0, 1)
+// inside it
+struct QueryCell {
+    int c0[3];
+    float f[3];
+};
+// a warp's shared memory: collected keys and the non-empty rows of a chunk
+struct QueryScratch {
+    float* key;
+    unsigned *id, *row_off;
+};
+struct Collected {
+    int cnt, rows;  // keys collected (-1: no search of this radius), rows read
+    unsigned seen;  // points of the rows read
+};
+
+// Collects every point within rad cells of a query. The cells of the ball are
+// walked by rows along x, one row a lane, clipped to the ball.
+// BOUNDED: where more than CAP points turn up, the k nearest so far are kept
+// and the bound falls to the k-th of them; nothing is collected (cnt 0) from
+// rows of more than `most` points. Otherwise the walk ends there, with a count
+// above CAP.
+template <int D, int CAP, bool BOUNDED>
+__device__ __forceinline__ Collected collect_ball(const CloudGrid& g, const unsigned* cell_start, const float4* sorted,
+                                                  const float* x, const QueryCell& q, float rad, int k,
+                                                  const QueryScratch& s, unsigned most = 0) {
+    const int lane = lane_id();
+    const unsigned below = (1u << lane) - 1u;
+    const float w = (float)g.w;
+    float T = (rad * w) * (rad * w);
+    // the ball in cells, with room for the rounding of T, dist^2 and f
+    const float rho = fmaf(rad, 1.f + 2e-5f, 1e-5f);
+    // T beyond FP32: distances that overflow tie at infinity, and only the
+    // shell walk sees all of them
+    if (!(rho < 1e4f && T < INFINITY)) return {-1, 0, 0u};
+    int a[3] = {0, 0, 0}, m[3] = {1, 1, 1};
+#pragma unroll
+    for (int d = 1; d < D; ++d) {
+        const int lo = max(q.c0[d] + (int)floorf(q.f[d] - rho), 0);
+        const int hi = min(q.c0[d] + (int)floorf(q.f[d] + rho), g.dims[d] - 1);
+        a[d] = lo;
+        m[d] = hi - lo + 1;
+    }
+    const int nrows = m[1] > 0 && m[2] > 0 ? m[1] * m[2] : 0;
+    if (nrows > 1024) return {-1, 0, 0u};
+    int cnt = 0;
+    unsigned seen = 0;
+    for (int t0 = 0; t0 < nrows && (BOUNDED || cnt <= CAP); t0 += 32) {
+        unsigned sb = 0, len = 0;
+        const int t = t0 + lane;
+        if (t < nrows) {
+            const int rz = D == 3 ? t / m[1] : 0, ry = t - rz * m[1];
+            const int cy = a[1] + ry, cz = a[2] + rz;
+            // squared distance of the row's slab in y (and z)
+            const float oy = (float)(cy - q.c0[1]) - q.f[1];
+            float e = fmaxf(0.f, fmaxf(oy, -1.f - oy));
+            float rem = fmaf(-e, e, rho * rho);
+            if (D == 3) {
+                const float oz = (float)(cz - q.c0[2]) - q.f[2];
+                e = fmaxf(0.f, fmaxf(oz, -1.f - oz));
+                rem = fmaf(-e, e, rem);
+            }
+            if (rem >= 0.f) {
+                const float hx = fmaf(sqrtf(rem), 1.f + 1e-5f, 1e-5f);
+                const int xa = max(q.c0[0] + (int)floorf(q.f[0] - hx), 0);
+                const int xb = min(q.c0[0] + (int)floorf(q.f[0] + hx), g.dims[0] - 1);
+                if (xa <= xb) {
+                    const int ca[3] = {xa, cy, cz};
+                    const int64_t ia = g.cell_base + cell_id<D>(g, ca);
+                    sb = cell_start[ia];
+                    len = cell_start[ia + (xb - xa) + 1] - sb;
+                }
+            }
+        }
+        unsigned incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const unsigned excl = incl - len, total = __shfl_sync(kFull, incl, 31);
+        if (BOUNDED) {
+            seen += total;
+            if (seen > most) return {0, nrows, seen};
+        }
+        // the non-empty rows in order: item i of the chunk is point
+        // row_off[rank of its row] + i
+        const unsigned some = __ballot_sync(kFull, len > 0);
+        if (len > 0) s.row_off[__popc(some & below)] = sb - excl;
+        __syncwarp();
+        int before = 0;  // rows begun in earlier batches
+        for (unsigned base = 0; base < total && (BOUNDED || cnt <= CAP); base += 32) {
+            const bool head = len > 0 && excl - base < 32u;
+            const unsigned heads = __reduce_or_sync(kFull, head ? 1u << (excl - base) : 0u);
+            const unsigned i = base + lane;
+            const int j = before + __popc(heads & (below | 1u << lane)) - 1;
+            before += __popc(heads);
+            float cd = INFINITY;
+            unsigned ci = 0xffffffffu;
+            if (i < total) {
+                const float4 v = sorted[s.row_off[j] + i];
+                const float sv[3] = {v.x, v.y, v.z};
+                cd = dist2_ref<D>(x, sv);
+                ci = __float_as_uint(v.w);
+            }
+            unsigned mask = __ballot_sync(kFull, cd <= T);
+            if (BOUNDED && cnt + __popc(mask) > CAP) {
+                __syncwarp();
+                T = keep_nearest<CAP / 32>(s.key, s.id, cnt, k);
+                cnt = k;
+                mask = __ballot_sync(kFull, cd <= T);
+            }
+            const int pos = cnt + __popc(mask & below);
+            if (cd <= T && pos < CAP) {
+                s.key[pos] = cd;
+                s.id[pos] = ci;
+            }
+            cnt += __popc(mask);
+        }
+        __syncwarp();
+    }
+    return {cnt, nrows, seen};
+}
+
+// the k nearest of cnt >= k collected keys
+template <int PER>
+__device__ __forceinline__ void write_nearest(const QueryScratch& s, int cnt, int k, uint32_t* out_idx, float* out_d2) {
+    float mine[PER];
+    unsigned who[PER];
+    int rank[PER];
+    rank_keys<PER>(s.key, s.id, cnt, mine, who, rank);
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+        if (lane_id() + 32 * u < cnt && rank[u] < k) {
+            out_idx[rank[u]] = who[u];
+            out_d2[rank[u]] = mine[u];
+        }
+    __syncwarp();
+}
+
+template <int R>
+struct QueryCap {
+    static constexpr int cap = 64 * R;  // keys collected at most: 32 R to keep, and a warp's more
+};
+
+// The search of a query whose first ball, of rad cells, held fewer than k
+// points or more than can be collected (rad 0: no first ball). A ball whose
+// rows hold far too many is shrunk before they are read (the first ones, and
+// one that grew well past a radius with too few); one with fewer than k grows.
+// A query that does not settle in kTries rounds or kRowsRead rows (an empty
+// neighbourhood, fewer points than k, a non-finite query) takes query_shells.
+constexpr int kTries = 8, kRowsRead = 4096;
+constexpr int kShrinks = 1;      // first rounds that may shrink the ball unread
+constexpr int kFarTooMany = 10;  // from this many times CAP points in its rows
+template <int D, int R>
+__device__ __noinline__ void query_again(float x0, float x1, float x2, const CloudGrid* grid, const unsigned* cell_start,
+                                         const float4* sorted, int k, float rad, QueryCell q, QueryScratch s,
+                                         uint32_t* out_idx, float* out_d2) {
+    constexpr int CAP = QueryCap<R>::cap;
+    const CloudGrid g = *grid;
+    const float x[3] = {x0, x1, x2};
+    float rad_lo = 0.f;  // the largest radius with too few
+    int rows = 0;
+    for (int tries = 0; rad > 0.f && tries < kTries && rows <= kRowsRead; ++tries) {
+        const bool may_shrink = tries < kShrinks || (rad_lo > 0.f && rad_lo < 0.6f * rad);
+        const unsigned most = may_shrink ? kFarTooMany * CAP : ~0u;
+        const Collected c = collect_ball<D, CAP, true>(g, cell_start, sorted, x, q, rad, k, s, most);
+        if (c.cnt < 0) break;
+        if (c.cnt >= k) {
+            write_nearest<CAP / 32>(s, c.cnt, k, out_idx, out_d2);
+            return;
+        }
+        rows += c.rows;
+        // to 1.4 k points by the count found, to 8 k or so by the rows' points
+        // (two fifths of them lie in the ball), halfway to a radius with too few
+        const bool shrink = c.seen > most;
+        const float r = (float)k * (shrink ? 20.f / (float)c.seen : 1.4f / fmaxf((float)c.cnt, 1.f));
+        const float step = D == 2 ? sqrtf(r) : cbrtf(r);
+        if (!shrink) rad_lo = rad;
+        rad = shrink ? fmaxf(rad * step, sqrtf(rad * rad_lo)) : rad * fminf(2.f, fmaxf(1.05f, step));
+    }
+    query_shells<D, R>(x0, x1, x2, grid, cell_start, sorted, k, out_idx, out_d2);
+}
+
 // Warp-per-query exact search by radius. R = 1 for k <= 32, 2 for k <= 64.
 //
 // The warp collects every point with dist^2 <= T in shared memory, T chosen
 // so that about 1.4 k points are expected, and ranks the collected (dist^2,
 // index) keys against each other: the k of lowest rank are the answer, since
-// no point outside the collection is closer than one inside. T starts from
-// the cloud's mean density, corrected for the part of the ball outside the
-// bounding box. Where more than CAP points turn up, the k nearest so far are
-// kept and T falls to the k-th one; a ball whose rows hold far more is shrunk
-// before they are read (the first ones, and one that grew well past a radius
-// with too few). Where fewer than k turn up the ball grows. A
-// query that does not settle in kTries rounds or kRowsRead rows (an empty
-// neighbourhood, fewer points than k, a non-finite query) takes query_shells.
+// no point outside the collection is closer than one inside. T comes from the
+// cloud's mean density, corrected for the part of the ball outside the
+// bounding box; a query that it does not suit goes on in query_again.
 //
-// The cells of the ball are walked by rows along x (one row a lane, clipped
-// to the ball), so a query reads ~2.5 k candidates instead of the ~8 k of
-// full cell shells, and ranking costs ~1.4 k broadcast reads instead of one
-// dependent insertion per improvement (64 clouds, 3.2 M points, k = 32:
-// 12.9 -> 4.4 ms; 250k points 0.98 -> 0.33 ms; 1 to 6 points a cell take the
-// same time within 10 %). Bound by instruction issue: ~1000 warp instructions
-// a query, 74 % of the issue slots, L1 38 %.
-//
+// A query reads ~2.5 k candidates instead of the ~8 k of full cell shells, and
+// ranking costs ~1.4 k broadcast reads instead of one dependent insertion per
+// improvement (64 clouds, 3.2 M points, k = 32: 12.9 -> 4.2 ms; 250k points
+// 0.98 -> 0.33 ms; 1 to 6 points a cell take the same time within 10 %). Bound
+// by instruction issue: ~1000 warp instructions a query, 74 % of the issue
+// slots, L1 38 %.
 // Clouds of uneven density, 30,000 points, all as queries: coordinates cubed
-// from a normal distribution 1.9 ms at k = 32 and 2.2 at 64, a box with half of
-// its points in a thousandth of it 0.32 and 0.52 (with a ball that was searched
-// again wherever too many points turned up 3.5, 4.7, 0.58 and 0.66; shells of
-// cells with sorted insertion 1.9, 2.5, 0.66, 1.1).
-// At most 64 registers for k <= 32: 4 blocks/SM, 4.67 -> 4.36 ms on the 64
-// clouds.
+// from a normal distribution, k = 8, 32, 64: 1.8, 1.7, 2.8 ms (searched again
+// wherever too many points turned up, with nothing kept: 3.0, 3.6, 4.7; shells
+// of cells with sorted insertion: 1.7, 1.8, 2.6).
+// The rare searches stand in a function of their own: in line they cost the
+// common one 5 to 7 %. 5 blocks/SM at 48 registers (4 at 64: 4.28 ms on the 64
+// clouds against 4.16, 3 at 80 4.74, 6 at 40 4.5).
 //
 // SELF: the queries are the sources; query q is the point at place q of the
 // cell order, so that a block's queries share cells.
-constexpr int kTries = 8, kRowsRead = 4096;
-constexpr int kShrinks = 2;      // first rounds that may shrink the ball unread
-constexpr int kFarTooMany = 10;  // from this many times CAP points in its rows
-template <int R>
-struct QueryCap {
-    static constexpr int cap = 64 * R;  // keys collected at most: 32 R to keep, and a warp's more
-};
 template <int D, int R, bool SELF>
-__global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float* qry, int64_t nq, const int64_t* q_offsets,
+__global__ void __launch_bounds__(256, 5) query_kernel(const float* qry, int64_t nq, const int64_t* q_offsets,
                                                     int q_nclouds, const CloudGrid* grids,
                                                     const unsigned* cell_start, const float4* sorted,
                                                     int k, uint32_t* out_idx, float* out_d2) {
-    constexpr int CAP = QueryCap<R>::cap, PER = CAP / 32;
+    constexpr int CAP = QueryCap<R>::cap;
     __shared__ __align__(16) float key_s[8][CAP + 4];
     __shared__ unsigned id_s[8][CAP];
     __shared__ unsigned row_s[8][32];
-    const int lane = lane_id(), wid = threadIdx.x >> 5;
-    float* const key = key_s[wid];
-    unsigned* const id = id_s[wid];
-    unsigned* const row_off = row_s[wid];
-    const unsigned below = (1u << lane) - 1u;
+    const int wid = threadIdx.x >> 5;
+    const QueryScratch scratch{key_s[wid], id_s[wid], row_s[wid]};
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < nq; p += warps) {
         const int cl = q_offsets ? find_cloud(q_offsets, q_nclouds, p) : 0;
@@ -478,10 +645,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float*
 #pragma unroll
             for (int d = 0; d < D; ++d) x[d] = qry[q * D + d];
         }
-        // in cells of the grid: cell c0 and the place f in [0, 1) inside it
-        const float w = (float)g.w;
-        int c0[3] = {0, 0, 0};
-        float f[3] = {0.f, 0.f, 0.f};
+        QueryCell c = {{0, 0, 0}, {0.f, 0.f, 0.f}};
         float out2 = 0.f;   // squared distance to the grid's box
         float inside = 1.f;  // part of the ball's box inside the grid's box
         const float r0 = g.r0;
@@ -491,138 +655,22 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3) query_kernel(const float*
             const double u = ((double)x[d] - g.lo[d]) * g.inv_w;
             ok = ok && fabs(u) < 1e9;
             const double fl = floor(u);
-            c0[d] = ok ? (int)fl : 0;
-            f[d] = (float)(u - fl);
+            c.c0[d] = ok ? (int)fl : 0;
+            c.f[d] = (float)(u - fl);
             const float uf = (float)u, hi = (float)g.dims[d];
             const float o = fmaxf(0.f, fmaxf(-uf, uf - hi));
             out2 = fmaf(o, o, out2);
             inside *= fmaxf(0.3f, (fminf(uf + r0, hi) - fmaxf(uf - r0, 0.f)) / (2.f * r0));
         }
         // radius in cells; past the box, the distance to it comes on top
-        float rad = fmaf(r0, exp2f((-1.f / D) * __log2f(inside)), sqrtf(out2));
-        float rad_lo = 0.f;  // the largest radius with too few
-        int rows_read = 0;
-        bool done = false;
-        for (int tries = 0; ok && tries < kTries; ++tries) {
-            float T = (rad * w) * (rad * w);
-            // the ball in cells, with room for the rounding of T, dist^2 and f
-            const float rho = fmaf(rad, 1.f + 2e-5f, 1e-5f);
-            // T beyond FP32: distances that overflow tie at infinity, and only
-            // the shell walk sees all of them
-            if (!(rho < 1e4f && T < INFINITY)) break;
-            int a[3] = {0, 0, 0}, m[3] = {1, 1, 1};
-#pragma unroll
-            for (int d = 1; d < D; ++d) {
-                const int lo = max(c0[d] + (int)floorf(f[d] - rho), 0);
-                const int hi = min(c0[d] + (int)floorf(f[d] + rho), g.dims[d] - 1);
-                a[d] = lo;
-                m[d] = hi - lo + 1;
-            }
-            const int nrows = m[1] > 0 && m[2] > 0 ? m[1] * m[2] : 0;
-            rows_read += nrows;
-            if (nrows > 1024 || rows_read > kRowsRead) break;
-            int cnt = 0;
-            unsigned seen = 0;  // points of the rows read
-            bool shrink = false;
-            for (int t0 = 0; t0 < nrows; t0 += 32) {
-                unsigned sb = 0, len = 0;
-                const int t = t0 + lane;
-                if (t < nrows) {
-                    const int rz = D == 3 ? t / m[1] : 0, ry = t - rz * m[1];
-                    const int cy = a[1] + ry, cz = a[2] + rz;
-                    // squared distance of the row's slab in y (and z)
-                    const float oy = (float)(cy - c0[1]) - f[1];
-                    float e = fmaxf(0.f, fmaxf(oy, -1.f - oy));
-                    float rem = fmaf(-e, e, rho * rho);
-                    if (D == 3) {
-                        const float oz = (float)(cz - c0[2]) - f[2];
-                        e = fmaxf(0.f, fmaxf(oz, -1.f - oz));
-                        rem = fmaf(-e, e, rem);
-                    }
-                    if (rem >= 0.f) {
-                        const float hx = fmaf(sqrtf(rem), 1.f + 1e-5f, 1e-5f);
-                        const int xa = max(c0[0] + (int)floorf(f[0] - hx), 0);
-                        const int xb = min(c0[0] + (int)floorf(f[0] + hx), g.dims[0] - 1);
-                        if (xa <= xb) {
-                            const int ca[3] = {xa, cy, cz};
-                            const int64_t ia = g.cell_base + cell_id<D>(g, ca);
-                            sb = cell_start[ia];
-                            len = cell_start[ia + (xb - xa) + 1] - sb;
-                        }
-                    }
-                }
-                unsigned incl = len;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned v = __shfl_up_sync(kFull, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const unsigned excl = incl - len, total = __shfl_sync(kFull, incl, 31);
-                seen += total;
-                shrink = seen > kFarTooMany * CAP && (tries < kShrinks || (rad_lo > 0.f && rad_lo < 0.6f * rad));
-                if (shrink) break;
-                // the non-empty rows in order: item i of the chunk is point
-                // row_off[rank of its row] + i
-                const unsigned some = __ballot_sync(kFull, len > 0);
-                if (len > 0) row_off[__popc(some & below)] = sb - excl;
-                __syncwarp();
-                int before = 0;  // rows begun in earlier batches
-                for (unsigned base = 0; base < total; base += 32) {
-                    const bool head = len > 0 && excl - base < 32u;
-                    const unsigned heads = __reduce_or_sync(kFull, head ? 1u << (excl - base) : 0u);
-                    const unsigned i = base + lane;
-                    const int j = before + __popc(heads & (below | 1u << lane)) - 1;
-                    before += __popc(heads);
-                    float cd = INFINITY;
-                    unsigned ci = 0xffffffffu;
-                    if (i < total) {
-                        const float4 s = sorted[row_off[j] + i];
-                        const float sv[3] = {s.x, s.y, s.z};
-                        cd = dist2_ref<D>(x, sv);
-                        ci = __float_as_uint(s.w);
-                    }
-                    unsigned mask = __ballot_sync(kFull, cd <= T);
-                    if (cnt + __popc(mask) > CAP) {
-                        __syncwarp();
-                        T = keep_nearest<PER>(key, id, cnt, k);
-                        cnt = k;
-                        mask = __ballot_sync(kFull, cd <= T);
-                    }
-                    if (cd <= T) {
-                        const int pos = cnt + __popc(mask & below);
-                        key[pos] = cd;
-                        id[pos] = ci;
-                    }
-                    cnt += __popc(mask);
-                }
-                __syncwarp();
-            }
-            if (!shrink && cnt >= k) {
-                float mine[PER];
-                unsigned who[PER];
-                int rank[PER];
-                rank_keys<PER>(key, id, cnt, mine, who, rank);
-#pragma unroll
-                for (int u = 0; u < PER; ++u)
-                    if (lane + 32 * u < cnt && rank[u] < k) {
-                        out_idx[q * k + rank[u]] = who[u];
-                        out_d2[q * k + rank[u]] = mine[u];
-                    }
-                __syncwarp();
-                done = true;
-                break;
-            }
-            __syncwarp();
-            // to 1.4 k points by the count found, to 8 k or so by the rows' points
-            // (two fifths of them lie in the ball), halfway to a radius with
-            // too few
-            const float s = (float)k * (shrink ? 20.f / (float)seen : 1.4f / fmaxf((float)cnt, 1.f));
-            const float step = D == 2 ? sqrtf(s) : cbrtf(s);
-            if (!shrink) rad_lo = rad;
-            rad = shrink ? fmaxf(rad * step, sqrtf(rad * rad_lo)) : rad * fminf(2.f, fmaxf(1.05f, step));
-        }
-        if (!done)
-            query_shells<D, R>(x[0], x[1], x[2], grids + cl, cell_start, sorted, k, out_idx + q * k, out_d2 + q * k);
+        const float rad = fmaf(r0, exp2f((-1.f / D) * __log2f(inside)), sqrtf(out2));
+        int cnt = -1;
+        if (ok) cnt = collect_ball<D, CAP, false>(g, cell_start, sorted, x, c, rad, k, scratch).cnt;
+        if (cnt >= k && cnt <= CAP)
+            write_nearest<CAP / 32>(scratch, cnt, k, out_idx + q * k, out_d2 + q * k);
+        else
+            query_again<D, R>(x[0], x[1], x[2], grids + cl, cell_start, sorted, k, cnt < 0 ? 0.f : rad, c, scratch,
+                              out_idx + q * k, out_d2 + q * k);
     }
 }
 
