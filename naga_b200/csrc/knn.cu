@@ -439,6 +439,7 @@ __device__ __forceinline__ Collected collect_ball(const CloudGrid& g, const unsi
     const unsigned below = (1u << lane) - 1u;
     const float w = (float)g.w;
     float T = (rad * w) * (rad * w);
+    unsigned Ti = 0xffffffffu;  // index bound of points at T itself
     // the ball in cells, with room for the rounding of T, dist^2 and f
     const float rho = fmaf(rad, 1.f + 2e-5f, 1e-5f);
     // T beyond FP32: distances that overflow tie at infinity, and only the
@@ -514,15 +515,18 @@ __device__ __forceinline__ Collected collect_ball(const CloudGrid& g, const unsi
                 cd = dist2_ref<D>(x, sv);
                 ci = __float_as_uint(v.w);
             }
-            unsigned mask = __ballot_sync(kFull, cd <= T);
+            bool take = BOUNDED ? cand_less(cd, ci, T, Ti) : cd <= T;
+            unsigned mask = __ballot_sync(kFull, take);
             if (BOUNDED && cnt + __popc(mask) > CAP) {
                 __syncwarp();
                 T = keep_nearest<CAP / 32>(s.key, s.id, cnt, k);
+                Ti = s.id[k - 1];
                 cnt = k;
-                mask = __ballot_sync(kFull, cd <= T);
+                take = cand_less(cd, ci, T, Ti);
+                mask = __ballot_sync(kFull, take);
             }
             const int pos = cnt + __popc(mask & below);
-            if (cd <= T && pos < CAP) {
+            if (take && pos < CAP) {
                 s.key[pos] = cd;
                 s.id[pos] = ci;
             }

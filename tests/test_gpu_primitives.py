@@ -57,6 +57,8 @@ def _awkward_cloud(kind, dim, rng):
         return p
     if kind == "stacks":  # 150 copies of each of 20 points: more ties than the collected keys
         return np.repeat(u(20), 150, 0)
+    if kind == "heaps":  # two places for all points: every batch a tie
+        return np.repeat(u(2), 2500, 0)
     if kind == "lattice":  # exact distance ties at every radius
         m = 14 if dim == 3 else 50
         return np.stack(np.meshgrid(*[np.arange(m)] * dim, indexing="ij"), -1).reshape(-1, dim) / 16.0
@@ -74,7 +76,7 @@ def _awkward_cloud(kind, dim, rng):
     return u(70)  # "few": barely more points than the largest k
 
 
-@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "lattice", "spike", "corner", "shell", "far", "vast",
+@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "heaps", "lattice", "spike", "corner", "shell", "far", "vast",
                                   "few"])
 @pytest.mark.parametrize("dim,k", [(2, 16), (3, 32), (3, 33), (2, 64), (3, 1)])
 def test_knn_awkward_clouds(naga, oracle, kind, dim, k):
