@@ -709,7 +709,8 @@ __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
 // first; cubic in 2-D, k = 16: 1.13, 1.03 and 1.05e-14). A query outside its
 // support (nearer to none than 0.6 of the farthest) would make a_r the larger
 // part: x is then the nearest support (30 spacings off, cubic: 1.3e-12, the
-// LU 2.5e-12). a_r is rounded to FP32 so that the sum of two is exact.
+// LU 2.5e-12). a_r is rounded to FP32, within its range, so that the sum of two
+// is exact.
 template <int D, int KC, int NR, class T>
 __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
     rbf_weights_gj_kernel(const float* __restrict__ src, int64_t nsrc, const uint32_t* __restrict__ support, int k,
@@ -759,7 +760,7 @@ __global__ void __launch_bounds__(32 * kGjBlockWarps, 4)
             }
             c = shape_fn(r2o, shape);
         }
-        const double al = (double)(float)c;
+        const double al = c < 1e30 ? (double)(float)c : c;
         if (lane < k) pr[lane] = al;  // solve() publishes its rows there later
         __syncwarp();
         S sys;

@@ -76,8 +76,8 @@ def _awkward_cloud(kind, dim, rng):
     return u(70)  # "few": barely more points than the largest k
 
 
-@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "heaps", "lattice", "spike", "corner", "shell", "far", "vast",
-                                  "few"])
+@pytest.mark.parametrize("kind", ["clusters", "sheet", "line", "stacks", "heaps", "lattice", "spike", "corner", "shell",
+                                  "far", "vast", "few"])
 @pytest.mark.parametrize("dim,k", [(2, 16), (3, 32), (3, 33), (2, 64), (3, 1)])
 def test_knn_awkward_clouds(naga, oracle, kind, dim, k):
     """Self and free queries (inside, beside and far outside the cloud)
@@ -354,6 +354,21 @@ def test_rbf_weights_round_no_more_than_an_lu(naga, dim, k, group, off):
         ref = ref + np.einsum("bij,bjk->bik", inv, b - np.einsum("bij,bjk->bik", A, ref))
     err = lambda y: np.median(np.linalg.norm(np.float64(y - ref[:, :k]), axis=1) / np.linalg.norm(np.float64(ref[:, :k]), axis=1))  # noqa: E731
     assert err(w.reshape(m, group, k).transpose(0, 2, 1)) <= 1.1 * err(lu[:, :k])
+
+
+@pytest.mark.parametrize("dim,k", [(2, 16), (3, 32)])
+def test_cubic_rbf_weights_do_not_depend_on_the_spacing(naga, dim, k):
+    """r^3 scales out of the system: spacings so small that the kernel's values
+    pass FP32's range (1e42), or so large that they vanish, give the weights of
+    spacing 1 up to the rounding of the systems (an LU's differ by 3e-12 on these
+    random clouds)."""
+    rng = np.random.default_rng(dim)
+    X = rng.random((15 ** dim, dim)).astype(np.float32) * 15
+    qry = rng.random((200, dim)) * 9 + 3
+    near = np.argsort(((X[None] - qry[:, None]) ** 2).sum(-1), 1)[:, :k].astype(np.int32)
+    ref, *others = (_np(naga.rbf_weights(_t(X), _t(near), _t(qry), 1, h, 1)) for h in (1.0, 2e-14, 1e-20, 1e12))
+    for w in others:
+        assert np.abs(w - ref).max() <= 1e-11 * np.abs(ref).max()
 
 
 @pytest.mark.parametrize("dim,shape,precision", [(2, 0, 0), (2, 1, 0), (3, 0, 0), (3, 1, 0), (3, 1, 1)])

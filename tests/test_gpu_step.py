@@ -347,6 +347,8 @@ def _runtime_calls(f):
         f()
         torch.cuda.synchronize()
     names = [e.name for e in prof.events()]
+    if not any(n.startswith("cuda") for n in names):
+        pytest.skip("no trace of CUDA runtime calls on this machine")
     return {n: names.count(n) for n in ("cudaGraphLaunch", "cudaStreamBeginCapture")}
 
 
