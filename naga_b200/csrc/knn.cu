@@ -12,8 +12,9 @@
 // cell); the points are counting-sorted by cell into float4 records
 // (x, y, z, local index). One warp serves one query. It gathers candidates
 // from contiguous row segments (cells along x are adjacent in the sorted
-// array): all rows its search ball touches, in query_kernel, or Chebyshev
-// shells of cells until no closer point can remain, in query_shells.
+// array): all rows its search ball touches, in query_kernel and, where the
+// first ball does not suit, query_again; or Chebyshev shells of cells until no
+// closer point can remain, in query_shells.
 #include "common.cuh"
 #include "scene_dev.hpp"
 #include "scratch.hpp"
@@ -624,9 +625,9 @@ __device__ __noinline__ void query_again(float x0, float x1, float x2, const Clo
 // cell order, so that a block's queries share cells.
 template <int D, int R, bool SELF>
 __global__ void __launch_bounds__(256, 5) query_kernel(const float* qry, int64_t nq, const int64_t* q_offsets,
-                                                    int q_nclouds, const CloudGrid* grids,
-                                                    const unsigned* cell_start, const float4* sorted,
-                                                    int k, uint32_t* out_idx, float* out_d2) {
+                                                       int q_nclouds, const CloudGrid* grids,
+                                                       const unsigned* cell_start, const float4* sorted,
+                                                       int k, uint32_t* out_idx, float* out_d2) {
     constexpr int CAP = QueryCap<R>::cap;
     __shared__ __align__(16) float key_s[8][CAP + 4];
     __shared__ unsigned id_s[8][CAP];
